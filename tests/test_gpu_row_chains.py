@@ -86,3 +86,62 @@ def test_backend_tools_run_and_verify_the_row_chains(tmp_path, name, init):
     v = subprocess.run([sys.executable, os.path.join(PKG, "bench", "verify.py"), "--out", dump, "--plan", plan, "--pattern", init, "--seed", "3",
                         "--rows", "0,1,2,3,7,15,31", "--rtol", "1e-5", "--atol", "1e-7"], capture_output=True, text=True)
     assert v.returncode == 0 and v.stdout.startswith("PASS"), v.stdout + v.stderr
+
+
+@pytest.mark.parametrize("dtype", ["f32", "f16"])
+@pytest.mark.parametrize("rows,N,ld,lead", [
+    (70, 1, 1, 0), (9, 7, 7, 3), (33, 31, 31, 1), (40, 63, 63, 0), (40, 65, 65, 5), (5, 127, 131, 2), (9, 257, 257, 0), (13, 1021, 1021, 7), (3, 2047, 2047, 0),
+    (3, 2049, 2049, 1), (7, 5003, 5003, 0), (3, 16383, 16383, 4), (2, 32767, 32767, 0), (3, 32769, 32769, 1), (2, 40000, 40000, 0),
+    (2, 65537, 65537, 0), (2, 150001, 150001, 3), (2, 300007, 300007, 0),
+])
+def test_row_chains_of_any_length_start_and_stride(wtc_lib, cuda_dev, rows, N, ld, lead, dtype):
+    """Rows that start anywhere: the element-wise ends, the short-row groups, one CTA, a cluster, and rows longer than a
+    cluster holds; input and output equally far from a 16-byte boundary, and not.  Nothing outside the rows is written."""
+    import ctypes as C
+    import torch
+    w = wtc_lib
+    rng = np.random.default_rng(rows + N)
+    t = torch.float16 if dtype == "f16" else torch.float32
+    X = (rng.standard_normal((rows, N)) * 2 + 0.5).astype(np.float16 if dtype == "f16" else np.float32)
+    src = torch.full((lead + rows * ld + 32,), 9.0, device=cuda_dev, dtype=t)
+    src[lead:lead + rows * ld].view(rows, ld)[:, :N] = torch.from_numpy(X).to(cuda_dev)
+    x64 = X.astype(np.float64)
+    e = np.exp(x64 - x64.max(axis=1, keepdims=True))
+    soft = e / e.sum(axis=1, keepdims=True)
+    var = np.repeat(((x64 - x64.mean(axis=1, keepdims=True)) ** 2).mean(axis=1, keepdims=True), N, axis=1)
+    for kind, ref in ((w.ROW_SOFTMAX, soft), (w.ROW_VARIANCE, var)):
+        for off in (lead, lead + 1):
+            out = torch.full((off + rows * ld + 32,), 9.0, device=cuda_dev, dtype=t)
+            d = w.RowChainDesc()
+            d.struct_size = C.sizeof(w.RowChainDesc)
+            d.kind, d.rows, d.N, d.ld_in, d.ld_out, d.dtype = kind, rows, N, ld, ld, w.F16 if dtype == "f16" else w.F32
+            d.mean_factor = d.var_factor = 1.0 / N
+            es = 2 if dtype == "f16" else 4
+            assert w.lib().wtc_row_chain_launch(C.byref(d), src.data_ptr() + lead * es, out.data_ptr() + off * es, w.current_stream_ptr()) == 0
+            torch.cuda.synchronize()
+            host = out.cpu().numpy().astype(np.float64)
+            assert (host[:off] == 9).all() and (host[off + rows * ld:] == 9).all()
+            got = host[off:off + rows * ld].reshape(rows, ld)
+            assert (got[:, N:] == 9).all()
+            # f16: the result's own rounding (2^-11, or half a subnormal step); f32: the exponent's rounding (2^-24 * |x - max| * log2 e
+            # < 2^-19.5 for |x - max| < 18) and the sums
+            tol = 2.0 ** -10 * np.abs(ref) + 2.0 ** -25 if dtype == "f16" else 4e-6 * np.abs(ref)
+            assert (np.abs(got[:, :N] - ref) <= tol).all(), (kind, off)
+
+
+def test_row_softmax_in_place_and_at_the_limits(wtc_lib, cuda_dev):
+    import torch
+    w = wtc_lib
+    for N in (61, 1021, 5003, 40000, 40001):
+        X = torch.randn((9, N), device=cuda_dev)
+        X[0] = torch.finfo(torch.float32).min                                   # a row of the type's lowest value: uniform
+        X[1, 5] = -float("inf")
+        X[2, 3] = float("nan")
+        X[3] = torch.finfo(torch.float32).min
+        X[3, 1] = 0.0
+        ref = torch.softmax(X.double(), dim=-1)
+        out = w.row_softmax(X, out=X)
+        assert out is X
+        for r in (0, 1, 3, 4, 8):
+            assert torch.allclose(out[r].double(), ref[r], rtol=4e-6, atol=0), (N, r)
+        assert torch.isnan(out[2]).all()
