@@ -101,14 +101,16 @@ template <bool F16> __device__ __forceinline__ uint4 load_raw(const void *base, 
 // does not.
 //
 // The exponent is fma(x, log2 e, -max * log2 e); (x - max) * log2 e in the ragged f32 form, which
-// stays exact at the maximum for rows near the type's limits.
+// stays exact at the maximum for rows near the type's limits.  KIND 2 is the
+// softmax of the f32 chain's logits (X and Out the same buffer): expf and a division, as the fused
+// f32 kernel computes them.
 template <int KIND, bool F16, int NV, bool RAGGED, bool PACKED, typename Reduce>
 __device__ __forceinline__ void chain_on_row(const void *X, void *Out, int64_t in0, int64_t out0, int N, int tid, int group, float c1, float c2,
                                              Reduce reduce) {
   static_assert(!PACKED || F16, "packed rows: f16");
   constexpr int V = VecOf<F16>::N;
-  constexpr float kFill = KIND == 0 ? -INFINITY : 0.f;
-  constexpr uint32_t kRawFill = KIND == 0 ? (F16 ? 0xFC00FC00u : 0xFF800000u) : 0u;      // the same as loaded bits
+  constexpr float kFill = KIND != 1 ? -INFINITY : 0.f;
+  constexpr uint32_t kRawFill = KIND != 1 ? (F16 ? 0xFC00FC00u : 0xFF800000u) : 0u;      // the same as loaded bits
   int head = 0, end = N;                        // whole vectors cover [head, end)
   if (RAGGED) {
     const int sh = static_cast<int>((reinterpret_cast<uintptr_t>(X) / (F16 ? 2 : 4) + static_cast<uint64_t>(in0)) & (V - 1));
@@ -136,7 +138,7 @@ __device__ __forceinline__ void chain_on_row(const void *X, void *Out, int64_t i
     if (PACKED) unpack_vec<F16>(raw[t], v[0]);
     return v[PACKED ? 0 : t];
   };
-  if (KIND == 0) {
+  if (KIND != 1) {
     float m = RAGGED ? fmaxf(xh, xt) : -INFINITY;
 #pragma unroll
     for (int t = 0; t < NV; ++t) {
@@ -147,7 +149,7 @@ __device__ __forceinline__ void chain_on_row(const void *X, void *Out, int64_t i
     }
     m = reduce(m, true);
     const float mb = m * kLog2e;
-    auto ex = [&](float x) { return RAGGED && !F16 ? ex2_approx((x - m) * kLog2e) : ex2_approx(fmaf(x, kLog2e, -mb)); };   // exp(x - max); -inf padding gives 0
+    auto ex = [&](float x) { return KIND == 2 ? expf(x - m) : RAGGED && !F16 ? ex2_approx((x - m) * kLog2e) : ex2_approx(fmaf(x, kLog2e, -mb)); };   // exp(x - max); -inf padding gives 0
     float s = 0.f;
     if (RAGGED) {
       xh = ex(xh); xt = ex(xt);
@@ -166,7 +168,7 @@ __device__ __forceinline__ void chain_on_row(const void *X, void *Out, int64_t i
     }
     s = reduce(s, false);
     const float inv = 1.0f / s;
-    auto norm = [&](float x) { return x * inv; };
+    auto norm = [&](float x) { return KIND == 2 ? x / s : x * inv; };
 #pragma unroll
     for (int t = 0; t < NV; ++t) {
       if (first + t * step < end) {
@@ -327,18 +329,18 @@ __global__ void __launch_bounds__(256) row_chain_block_kernel(const void *X, voi
                                                               int64_t ld_out, float c1, float c2) {
   __shared__ float scratch[32];
   const int64_t in0 = static_cast<int64_t>(blockIdx.x) * ld_in, out0 = static_cast<int64_t>(blockIdx.x) * ld_out;
-  if (KIND == 0) {
+  if (KIND != 1) {
     float m = -INFINITY;
     for (int j = threadIdx.x; j < N; j += blockDim.x) m = fmaxf(m, load_elem<IN16>(X, in0 + j));
     m = block_reduce(m, true, scratch);
-    auto ex = [&](float x) { return ex2_approx((x - m) * kLog2e); };
+    auto ex = [&](float x) { return KIND == 2 ? expf(x - m) : ex2_approx((x - m) * kLog2e); };
     float s = 0.f;
     for (int j = threadIdx.x; j < N; j += blockDim.x) s += ex(load_elem<IN16>(X, in0 + j));
     s = block_reduce(s, false, scratch);
     const float inv = 1.0f / s;
     for (int j = threadIdx.x; j < N; j += blockDim.x) {
       const float y = ex(load_elem<IN16>(X, in0 + j));
-      store_elem<OUT16>(Out, out0 + j, y * inv);
+      store_elem<OUT16>(Out, out0 + j, KIND == 2 ? y / s : y * inv);
     }
   } else {
     float s = 0.f;
@@ -434,6 +436,7 @@ cudaError_t launch_row_chain(int kind, const void *X, void *Out, int64_t rows, i
   if (N > 0x7fffffff) return cudaErrorInvalidValue;
   if ((in_f16 != 0) != (out_f16 != 0)) return cudaErrorInvalidValue;
   const int n = static_cast<int>(N);
+  if (kind == 2 && !in_f16) return launch_typed<2, false>(X, Out, rows, n, ld_in, ld_out, c1, c2, s);
   if (kind == 0) return in_f16 ? launch_typed<0, true>(X, Out, rows, n, ld_in, ld_out, c1, c2, s) : launch_typed<0, false>(X, Out, rows, n, ld_in, ld_out, c1, c2, s);
   if (kind == 1) return in_f16 ? launch_typed<1, true>(X, Out, rows, n, ld_in, ld_out, c1, c2, s) : launch_typed<1, false>(X, Out, rows, n, ld_in, ld_out, c1, c2, s);
   return cudaErrorInvalidValue;

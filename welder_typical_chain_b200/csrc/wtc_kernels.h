@@ -93,7 +93,8 @@ cudaError_t launch_softmax_passes(const float *C32, float *E, float *mx, float *
                                   int N, int64_t ldo, int64_t o_batch_stride, int out_f16, cudaStream_t s);
 
 // Row-only chains (row_chain_kernels.cu).  kind 0: Out = softmax_row(X); kind 1: Out[i, :] =
-// c2 * sum_j (X[i,j] - c1 * sum_j X[i,j])^2.  Row strides in elements.
+// c2 * sum_j (X[i,j] - c1 * sum_j X[i,j])^2; kind 2 (f32): softmax_row of the f32 chain's logits,
+// with the exponential and division of the fused f32 kernel.  Row strides in elements; X and Out may be the same buffer.
 cudaError_t launch_row_chain(int kind, const void *X, void *Out, int64_t rows, int64_t N, int64_t ld_in, int64_t ld_out, int in_f16,
                              int out_f16, float c1, float c2, cudaStream_t s);
 
@@ -107,6 +108,7 @@ struct SimtParams {
   float scale;
 };
 cudaError_t launch_simt_fused(const void *A, const void *B, void *Out, const SimtParams &p, cudaStream_t s);
+int simt_fused_launches(const SimtParams &p);
 // Unfused five-kernel pipeline: matmul -> row max -> exp -> row sum -> divide,
 // with C32[M,N], max[M], E[M,N], sum[M] in global memory (workspace).
 cudaError_t launch_simt_unfused(const void *A, const void *B, void *Out, void *workspace, const SimtParams &p,

@@ -76,6 +76,17 @@ size_t align256(size_t v) { return (v + 255) & ~static_cast<size_t>(255); }
 
 bool mult8(int64_t v) { return (v & 7) == 0; }
 
+wtc::SimtParams simt_params(const Resolved &r) {
+  wtc::SimtParams s;
+  s.batch = r.d.batch; s.M = (int)r.d.M; s.N = (int)r.d.N; s.K = (int)r.d.K;
+  s.lda = r.d.lda; s.ldb = r.d.ldb; s.ldo = r.d.ldo;
+  s.a_batch_stride = r.d.a_batch_stride; s.b_batch_stride = r.d.b_batch_stride; s.o_batch_stride = r.d.o_batch_stride;
+  s.in_f16 = r.d.in_dtype == WTC_F16; s.out_f16 = r.d.out_dtype == WTC_F16;
+  s.acc_mode = r.d.acc_dtype == WTC_F16 ? 1 : 0;
+  s.scale = r.d.scale;
+  return s;
+}
+
 int resolve(const wtc_chain_desc *in, Resolved &r) {
   if (!in) return fail(WTC_E_ARG, "null descriptor");
   if (in->struct_size != static_cast<int32_t>(sizeof(wtc_chain_desc)))
@@ -219,7 +230,7 @@ int resolve(const wtc_chain_desc *in, Resolved &r) {
     }
   } else {
     p.kernel = WTC_KERNEL_SIMT_FUSED;
-    p.launches = (d.M > 0 && d.N > 0) ? 1 : 0;
+    p.launches = (d.M > 0 && d.N > 0) ? wtc::simt_fused_launches(simt_params(r)) : 0;
     p.threads = 256;
     p.tile_m = 16; p.tile_n = static_cast<int32_t>(d.N); p.tile_k = 64;
   }
@@ -355,17 +366,6 @@ int status_result(int v) {
 }
 
 bool aligned16(const void *p) { return (reinterpret_cast<uintptr_t>(p) & 15) == 0; }
-
-wtc::SimtParams simt_params(const Resolved &r) {
-  wtc::SimtParams s;
-  s.batch = r.d.batch; s.M = (int)r.d.M; s.N = (int)r.d.N; s.K = (int)r.d.K;
-  s.lda = r.d.lda; s.ldb = r.d.ldb; s.ldo = r.d.ldo;
-  s.a_batch_stride = r.d.a_batch_stride; s.b_batch_stride = r.d.b_batch_stride; s.o_batch_stride = r.d.o_batch_stride;
-  s.in_f16 = r.d.in_dtype == WTC_F16; s.out_f16 = r.d.out_dtype == WTC_F16;
-  s.acc_mode = r.d.acc_dtype == WTC_F16 ? 1 : 0;
-  s.scale = r.d.scale;
-  return s;
-}
 
 // mode: 0 whole chain, 1 partial (leave un-normalised values + row stats)
 int launch_resolved(Resolved &r, const void *A, const void *B, void *Out, void *ws, size_t ws_bytes, void *row_stats,
