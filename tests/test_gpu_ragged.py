@@ -1,0 +1,151 @@
+"""f16 chains whose rows TMA cannot take (strides that are no multiple of 16 bytes): padded operand
+copies, tensor-core contraction, output rows written from the staging tiles; against the CPU checker,
+and against the SIMT kernel, which stays the path of a call without workspace or 16-byte pointers."""
+import ctypes as C
+
+import numpy as np
+import pytest
+
+from oracle import oracle
+
+
+def _operands(batch, M, N, K, shared=False, seed=0):
+    A = oracle.normal((batch, M, K) if batch > 1 else (M, K), 100 + seed)
+    B = oracle.normal((batch, K, N) if batch > 1 and not shared else (K, N), 200 + seed)
+    return A, B
+
+
+def _ref(A, B, scale):
+    if A.ndim == 2:
+        return oracle.chain(A, B, scale)
+    return np.stack([oracle.chain(A[i], B[i] if B.ndim == 3 else B, scale) for i in range(A.shape[0])])
+
+
+def test_ragged_plans(wtc_lib):
+    """Which copies a shape needs; small shapes and rows the SIMT kernel does not take stay as they were."""
+    w = wtc_lib
+    for (M, N, K), copies, extra in [((1000, 333, 64), "B", 1), ((1000, 328, 61), "A", 1), ((1000, 333, 61), "AB", 1), ((4000, 2305, 64), "B", 1)]:
+        p = w.plan_query(w.make_desc(1, M, N, K))
+        tiled = N > 2048
+        want = 0
+        if "A" in copies:
+            want += -(-M * (-(-K // 8) * 8) * 2 // 256) * 256
+        if "B" in copies:
+            want += -(-K * (-(-N // 64) * 64) * 2 // 256) * 256
+        if tiled:
+            want += M * -(-N // 256) * 8
+        assert p.kernel == (w.KERNEL_TC_TILED if tiled else w.KERNEL_TC_CLUSTER)
+        assert p.launches == (2 if tiled else 1) + extra and p.workspace_bytes == want
+    # padded strides: nothing to copy
+    p = w.plan_query(w.make_desc(1, 1000, 333, 64, ldb=336, ldo=336))
+    assert p.kernel == w.KERNEL_TC_CLUSTER and p.launches == 1 and p.workspace_bytes == 0
+    assert w.plan_query(w.make_desc(1, 100, 70, 64)).kernel == w.KERNEL_SIMT_FUSED
+    assert w.plan_query(w.make_desc(1, 1000, 333, 64, flags=w.FLAG_FORCE_SIMT)).kernel == w.KERNEL_SIMT_FUSED
+    assert w.plan_query(w.make_desc(1, 500, 60001, 64)).kernel == w.KERNEL_SIMT_FUSED      # refused at launch, as before
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("batch,M,N,K,out,kw", [
+    (1, 2000, 129, 64, "f16", {}),          # 128-column tiles, one column in the second
+    (1, 4000, 127, 33, "f16", {}),          # narrower than a tile, ragged K
+    (1, 8200, 255, 63, "f32", {}),          # f32 probabilities, 256-column tile
+    (4, 1021, 1021, 64, "f16", {}),
+    (24, 1021, 1021, 64, "f16", {}),        # relay: several tiles per CTA, two operand stages
+    (24, 700, 1001, 251, "f16", {}),        # relay with three stages, ragged K
+    (24, 700, 1001, 251, "f16", {"shared": True}),
+    (3, 200, 2047, 72, "f32", {}),          # full cluster of eight
+    (1, 257, 2049, 64, "f16", {}),          # tiled: one column in the ninth tile
+    (2, 300, 3001, 100, "f16", {}),         # tiled, ragged row rescale across tile borders
+    (1, 300, 3001, 100, "f32", {}),
+    (1, 700, 520, 61, "f16", {}),           # only A is copied: TMA stores
+    (1, 700, 1025, 64, "f16", {"acc_dtype": "F16"}),
+])
+def test_ragged_matches_the_checker(wtc_lib, cuda_dev, batch, M, N, K, out, kw):
+    import torch
+    w = wtc_lib
+    A, B = _operands(batch, M, N, K, kw.get("shared", False))
+    tA, tB = torch.from_numpy(A).to(cuda_dev), torch.from_numpy(B).to(cuda_dev)
+    acc = getattr(w, kw.get("acc_dtype", "F32"))
+    scale = 0.9 / np.sqrt(K)
+    odt = w.F16 if out == "f16" else w.F32
+    d = w.make_desc(batch, M, N, K, out_dtype=odt, acc_dtype=acc, shared_b=kw.get("shared", False))
+    assert w.plan_query(d).kernel in (w.KERNEL_TC_CLUSTER, w.KERNEL_TC_TILED)
+    got = w.matmul_softmax(tA, tB, scale, out_dtype=odt, acc_dtype=acc)
+    w.check_device_status()
+    got = got.cpu().numpy()
+    if acc == w.F32:
+        r = oracle.compare(got.reshape(-1, N), _ref(A, B, scale).reshape(-1, N))
+        assert r["ok"], r
+    simt = w.matmul_softmax(tA, tB, scale, out_dtype=odt, acc_dtype=acc, flags=w.FLAG_FORCE_SIMT).cpu().numpy().astype(np.float64)
+    # both round the same f32 sums (differing by their order) to the output type: one ulp of it apart (2^-10 relative; two for the
+    # tiled form, which rounds twice), and with an f16 matmul result one ulp of a logit (2^-10 relative, |logit| < 8) besides
+    tol = (2.0 ** -9 if out == "f16" else 2e-5) + (2.0 ** -7 if acc == w.F16 else 0)
+    assert (np.abs(got.astype(np.float64) - simt) <= tol * simt + 2.0 ** -23).all()
+
+
+@pytest.mark.gpu
+def test_ragged_strided_output_and_neighbours(wtc_lib, cuda_dev):
+    """A padded output: the columns between rows, and what lies before and behind, stay untouched; odd row starts."""
+    import torch
+    w = wtc_lib
+    M, N, K = 300, 1021, 64
+    A, B = _operands(1, M, N, K)
+    tA, tB = torch.from_numpy(A).to(cuda_dev), torch.from_numpy(B).to(cuda_dev)
+    for ldo, lead in [(1021, 1), (1023, 0), (1030, 3), (1024, 8)]:
+        d = w.make_desc(1, M, N, K, scale=0.1, ldo=ldo)
+        buf = torch.full((lead + M * ldo + 64,), 7.0, device=cuda_dev, dtype=torch.float16)
+        ws = torch.empty(max(16, w.workspace_bytes(d)), device=cuda_dev, dtype=torch.uint8)
+        rc = w.lib().wtc_matmul_softmax_launch(C.byref(d), tA.data_ptr(), tB.data_ptr(), buf.data_ptr() + 2 * lead, ws.data_ptr(), ws.numel(),
+                                               w.current_stream_ptr(), None)
+        assert rc == 0
+        w.check_device_status()
+        host = buf.cpu().numpy()
+        assert (host[:lead] == 7).all() and (host[lead + M * ldo:] == 7).all()
+        rows = host[lead:lead + M * ldo].reshape(M, ldo)
+        assert (rows[:, N:] == 7).all()
+        r = oracle.compare(rows[:, :N], oracle.chain(A, B, 0.1))
+        assert r["ok"], r
+
+
+@pytest.mark.gpu
+def test_ragged_without_workspace_or_alignment(wtc_lib, cuda_dev):
+    """A call that brings no workspace, and one whose operands start off a 16-byte boundary, still run."""
+    import torch
+    w = wtc_lib
+    M, N, K = 300, 1021, 64
+    A, B = _operands(1, M, N, K)
+    ref = oracle.chain(A, B, 0.1)
+    tB = torch.from_numpy(B).to(cuda_dev)
+    store = torch.empty(M * K + 8, device=cuda_dev, dtype=torch.float16)
+    for lead in (0, 1):
+        tA = store[lead:lead + M * K].view(M, K)
+        tA.copy_(torch.from_numpy(A).to(cuda_dev))
+        d = w.make_desc(1, M, N, K, scale=0.1)
+        out = torch.empty((M, N), device=cuda_dev, dtype=torch.float16)
+        ws = torch.empty(w.workspace_bytes(d), device=cuda_dev, dtype=torch.uint8)
+        for ptr, size in ((None, 0), (ws.data_ptr(), ws.numel())):
+            out.zero_()
+            rc = w.lib().wtc_matmul_softmax_launch(C.byref(d), tA.data_ptr(), tB.data_ptr(), out.data_ptr(), ptr, size, w.current_stream_ptr(), None)
+            assert rc == 0
+            w.check_device_status()
+            r = oracle.compare(out.cpu().numpy(), ref)
+            assert r["ok"], (lead, size, r)
+
+
+@pytest.mark.gpu
+def test_rounded_f32_operands_of_ragged_shape(wtc_lib, cuda_dev):
+    """f32 arguments truncated to f16, K and N no multiples of 8: the rounded copies have padded rows.  Same contraction
+    as the f16 operands' own ragged path, so the same bits."""
+    import torch
+    w = wtc_lib
+    rng = np.random.default_rng(3)
+    for batch, M, N, K in ((1, 700, 1001, 251), (3, 300, 333, 100)):
+        A = rng.standard_normal((batch, M, K) if batch > 1 else (M, K)).astype(np.float32)
+        B = rng.standard_normal((K, N)).astype(np.float32)
+        got = w.matmul_softmax(torch.from_numpy(A).to(cuda_dev), torch.from_numpy(B).to(cuda_dev), 0.1, out_dtype=w.F16, flags=w.FLAG_MATMUL_F16)
+        w.check_device_status()
+        A16, B16 = A.astype(np.float16), B.astype(np.float16)
+        same = w.matmul_softmax(torch.from_numpy(A16).to(cuda_dev), torch.from_numpy(B16).to(cuda_dev), 0.1)
+        assert torch.equal(got, same)
+        r = oracle.compare(got.cpu().numpy().reshape(-1, N), _ref(A16, B16, 0.1).reshape(-1, N))
+        assert r["ok"], r

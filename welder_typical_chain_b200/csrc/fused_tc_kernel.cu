@@ -40,6 +40,8 @@
 //               fourth operand stage.
 // PAIR: two CTAs issue one 256-row tcgen05 cta_group::2 MMA (tiled flavour, long K).
 // OUT32: f32 probabilities.
+// DIRECT: output rows that TMA cannot store (a stride that is no multiple of 16 bytes): the warp
+// that staged a tile writes its rows itself (split form).
 // KD, TM: K depth of a pipeline stage (64; 32 or 128 on request) and rows of a tile (128;
 // 64 on request, tcgen05.mma with M = 64) -- the schedule's tileK and tileM.
 //
@@ -136,6 +138,53 @@ __device__ __forceinline__ void stage_row_f32(uint8_t *tile, int lane, const flo
   }
 }
 
+// A staged tile (32 rows of 128 bytes: 64 f16 or 32 f32 columns, 128-byte swizzle) to rows that start
+// anywhere.  Few warps store and each issues one dependent instruction in about four clocks, so what
+// counts is instructions a row: a 4-byte word a lane (f16 words put together from two staged ones
+// where the row starts on an odd element -- the same lanes, offsets and shifts for every other row),
+// ROWS rows in flight; the single elements that are left in front and behind go last, a row a lane.
+// (16-byte pieces, shifted together by each lane, took 57 us for 24504 x 1021 x 64, this takes 42.)
+// Whole warps; the tile may be overwritten when the call returns.
+template <bool F32, int ROWS>
+__device__ __forceinline__ void store_tile_direct(const uint8_t *tile, const TcParams &p, int lane, int b, int row0, int col0) {
+  constexpr int ES = F32 ? 4 : 2;
+  const int cols = min(p.N - col0, 128 / ES);
+  const int rows = min(32, p.M - row0);
+  const int64_t ld = p.ldo * ES;
+  char *out = static_cast<char *>(p.out) + (b * p.o_batch_stride + static_cast<int64_t>(row0) * p.ldo + col0) * ES;
+  // rows of even and of odd number: does the row start on an odd element, this lane's word, whether it exists
+  const uint32_t odd0 = F32 ? 0u : static_cast<uint32_t>(reinterpret_cast<uintptr_t>(out) >> 1) & 1u;
+  const uint32_t odd1 = F32 ? 0u : odd0 ^ (static_cast<uint32_t>(p.ldo) & 1u);
+  char *mine0 = out + lane * 4 + odd0 * 2, *mine1 = out + ld + lane * 4 + odd1 * 2;
+  const bool word0 = F32 ? lane < cols : 2 * lane + 1 + static_cast<int>(odd0) < cols;
+  const bool word1 = F32 ? lane < cols : 2 * lane + 1 + static_cast<int>(odd1) < cols;
+#pragma unroll 1
+  for (int r0 = 0; r0 < rows; r0 += ROWS) {
+    uint32_t w[ROWS];
+#pragma unroll
+    for (int u = 0; u < ROWS; ++u) w[u] = *reinterpret_cast<const uint32_t *>(tile + (r0 + u) * 128 + ((lane * 4) ^ (((r0 + u) & 7) << 4)));
+    if (!F32) {
+#pragma unroll
+      for (int u = 0; u < ROWS; ++u) w[u] = __funnelshift_r(w[u], __shfl_down_sync(0xffffffffu, w[u], 1), (u & 1 ? odd1 : odd0) * 16);
+    }
+#pragma unroll
+    for (int u = 0; u < ROWS; u += 2) {
+      if (word0 && r0 + u < rows) *reinterpret_cast<uint32_t *>(mine0) = w[u];
+      if (word1 && r0 + u + 1 < rows) *reinterpret_cast<uint32_t *>(mine1) = w[u + 1];
+      mine0 += 2 * ld; mine1 += 2 * ld;
+    }
+  }
+  if (!F32 && lane < rows) {
+    const bool odd = lane & 1 ? odd1 : odd0;
+    char *row = out + lane * ld;
+    const uint8_t *src = tile + lane * 128;
+    if (odd) *reinterpret_cast<uint16_t *>(row) = *reinterpret_cast<const uint16_t *>(src + ((lane & 7) << 4));
+    if ((cols - (odd ? 1 : 0)) & 1)
+      *reinterpret_cast<uint16_t *>(row + (cols - 1) * 2) = *reinterpret_cast<const uint16_t *>(src + (((cols - 1) * 2) ^ ((lane & 7) << 4)));
+  }
+  __syncwarp();
+}
+
 // Bring-up builds (-DWTC_BRINGUP) stamp the phases of each CTA's first tile; the default
 // build carries no stamps.
 #ifdef WTC_BRINGUP
@@ -207,7 +256,7 @@ __device__ __forceinline__ void scale_pack(const uint32_t (&r)[32], float f, uin
   for (int i = 0; i < 32; i += 2) h[i >> 1] = pack_f16x2(__uint_as_float(r[i]) * f, __uint_as_float(r[i + 1]) * f);
 }
 
-template <int BN, int STAGES, bool CLUSTER, int EPI, bool PAIR, bool OUT32, int KD, int TM>
+template <int BN, int STAGES, bool CLUSTER, int EPI, bool PAIR, bool OUT32, int KD, int TM, bool DIRECT>
 __global__ void __launch_bounds__(kThreadsFor(EPI), 1)
 fused_tc_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CUtensorMap tmB,
                 const __grid_constant__ CUtensorMap tmO, const TcParams p) {
@@ -223,6 +272,7 @@ fused_tc_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__
   static_assert(!(RELAY || SINGLE) || (CLUSTER && !PAIR && !OUT32 && BN == 256 && TM == 128), "sixteen-warp epilogues: cluster flavour, 128 x 256 tiles, f16 staged stores");
   static_assert(!OUT32 || !PAIR, "f32 output: unpaired CTAs");
   static_assert(!PAIR || !CLUSTER, "CTA pairs: tiled flavour only");
+  static_assert(!DIRECT || (!PAIR && EPI == EPI_SPLIT && KD == kTcBlockK && TM == kTcBlockM), "rows written by threads: split form, default tiles");
   // The 128-byte swizzle needs the stage buffers on 1024-byte boundaries.  There is no
   // static shared memory in this kernel, so the dynamic window starts aligned; if it ever
   // does not, every thread leaves before any barrier or TMEM state exists.
@@ -968,9 +1018,11 @@ fused_tc_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__
 #pragma unroll
             for (int i = 0; i < 32; ++i) { v[i] = __uint_as_float(r[c][i]) * f; if (!CLUSTER) sum_r += v[i]; }
             stage_row_f32(tile, lane, v);
-            fence_proxy_async_smem();
+            if (!DIRECT) fence_proxy_async_smem();
             __syncwarp();
-            if (lane == 0) {
+            if (DIRECT) {
+              if (rows_live) store_tile_direct<true, 8>(tile, p, lane, b, row0, col0 + c * 32);
+            } else if (lane == 0) {
               if (rows_live) tma_store_3d(&tmO, tile, col0 + c * 32, row0, b);
               tma_store_commit();
             }
@@ -994,9 +1046,15 @@ fused_tc_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__
             stage_row_chunk(stg + (c >> 1) * 4096, lane, c & 1, h);
           }
         }
-        fence_proxy_async_smem();
+        if (!DIRECT) fence_proxy_async_smem();
         __syncwarp();
-        if (lane == 0) {
+        if (DIRECT) {
+          if (rows_live) {
+#pragma unroll
+            for (int g = 0; g < NCH / 2; ++g)
+              if (g * 64 < valid) store_tile_direct<false, 8>(stg + g * 4096, p, lane, b, row0, col0 + g * 64);
+          }
+        } else if (lane == 0) {
           if (rows_live) {
 #pragma unroll
             for (int g = 0; g < NCH / 2; ++g)
@@ -1022,9 +1080,11 @@ fused_tc_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__
               }
               stage_row_chunk(stg, lane, hc, h);
             }
-            fence_proxy_async_smem();
+            if (!DIRECT) fence_proxy_async_smem();
             __syncwarp();
-            if (lane == 0) {
+            if (DIRECT) {
+              if (rows_live) store_tile_direct<false, 8>(stg, p, lane, b, row0, col0 + g * 64);
+            } else if (lane == 0) {
               if (rows_live) tma_store_3d(&tmO, stg, col0 + g * 64, row0, b);
               tma_store_commit();
             }
@@ -1071,11 +1131,11 @@ struct DeviceFacts {
   int registers = 0;
 };
 
-template <int BN, int STAGES, bool CLUSTER, int EPI, bool PAIR, bool OUT32, int KD, int TM>
+template <int BN, int STAGES, bool CLUSTER, int EPI, bool PAIR, bool OUT32, int KD, int TM, bool DIRECT>
 cudaError_t launch_impl(const CUtensorMap &tmA, const CUtensorMap &tmB, const CUtensorMap &tmO, TcParams p,
                         int cluster_n, int num_sms, cudaStream_t s, TcLaunchInfo *info) {
   using L = SmemLayout<BN, STAGES, CLUSTER, EPI, PAIR, OUT32, KD, TM>;
-  auto kern = fused_tc_kernel<BN, STAGES, CLUSTER, EPI, PAIR, OUT32, KD, TM>;
+  auto kern = fused_tc_kernel<BN, STAGES, CLUSTER, EPI, PAIR, OUT32, KD, TM, DIRECT>;
   static DeviceFacts facts[64];   // per template instance, per device
   int dev = 0;
   cudaError_t e = cudaGetDevice(&dev);
@@ -1141,25 +1201,30 @@ cudaError_t launch_impl(const CUtensorMap &tmA, const CUtensorMap &tmB, const CU
 
 } // namespace
 
-// Every instantiated variant, once: X(BN, STAGES, CLUSTER, EPI, PAIR, OUT32, KD, TM).
+// Every instantiated variant, once: X(BN, STAGES, CLUSTER, EPI, PAIR, OUT32, KD, TM, DIRECT).
 #define WTC_TC_VARIANTS(X)                                                                                \
-  X(128, 4, true, EPI_SPLIT, false, true, 64, 128) X(kTcBlockN, 3, true, EPI_SPLIT, false, true, 64, 128)            \
-  X(128, 4, true, EPI_SPLIT, false, false, 64, 128) X(kTcBlockN, 3, true, EPI_SPLIT, false, false, 64, 128)          \
-  X(kTcBlockN, 2, true, EPI_RELAY, false, false, 64, 128) X(kTcBlockN, 3, true, EPI_RELAY, false, false, 64, 128)    \
-  X(kTcBlockN, 4, true, EPI_SINGLE, false, false, 64, 128)                                                      \
-  X(128, 6, false, EPI_SPLIT, false, true, 64, 128) X(kTcBlockN, 4, false, EPI_SPLIT, false, true, 64, 128)          \
-  X(128, 6, false, EPI_SPLIT, false, false, 64, 128) X(kTcBlockN, 4, false, EPI_SPLIT, false, false, 64, 128)        \
-  X(kTcBlockN, 6, false, EPI_SPLIT, true, false, 64, 128)                                                       \
+  X(128, 4, true, EPI_SPLIT, false, true, 64, 128, false) X(kTcBlockN, 3, true, EPI_SPLIT, false, true, 64, 128, false)            \
+  X(128, 4, true, EPI_SPLIT, false, false, 64, 128, false) X(kTcBlockN, 3, true, EPI_SPLIT, false, false, 64, 128, false)          \
+  X(kTcBlockN, 2, true, EPI_RELAY, false, false, 64, 128, false) X(kTcBlockN, 3, true, EPI_RELAY, false, false, 64, 128, false)    \
+  X(kTcBlockN, 4, true, EPI_SINGLE, false, false, 64, 128, false)                                                      \
+  X(128, 6, false, EPI_SPLIT, false, true, 64, 128, false) X(kTcBlockN, 4, false, EPI_SPLIT, false, true, 64, 128, false)          \
+  X(128, 6, false, EPI_SPLIT, false, false, 64, 128, false) X(kTcBlockN, 4, false, EPI_SPLIT, false, false, 64, 128, false)        \
+  X(kTcBlockN, 6, false, EPI_SPLIT, true, false, 64, 128, false)                                                       \
   /* other stage depths (the schedule's tileK): eight-warp epilogue, f16 output */                        \
-  X(128, 8, true, EPI_SPLIT, false, false, 32, 128) X(kTcBlockN, 6, true, EPI_SPLIT, false, false, 32, 128)          \
-  X(128, 12, false, EPI_SPLIT, false, false, 32, 128) X(kTcBlockN, 8, false, EPI_SPLIT, false, false, 32, 128)       \
-  X(128, 2, true, EPI_SPLIT, false, false, 128, 128)                                                            \
-  X(128, 3, false, EPI_SPLIT, false, false, 128, 128) X(kTcBlockN, 2, false, EPI_SPLIT, false, false, 128, 128)       \
+  X(128, 8, true, EPI_SPLIT, false, false, 32, 128, false) X(kTcBlockN, 6, true, EPI_SPLIT, false, false, 32, 128, false)          \
+  X(128, 12, false, EPI_SPLIT, false, false, 32, 128, false) X(kTcBlockN, 8, false, EPI_SPLIT, false, false, 32, 128, false)       \
+  X(128, 2, true, EPI_SPLIT, false, false, 128, 128, false)                                                            \
+  X(128, 3, false, EPI_SPLIT, false, false, 128, 128, false) X(kTcBlockN, 2, false, EPI_SPLIT, false, false, 128, 128, false)       \
   /* 64-row tiles (the schedule's tileM = 64), stage depth 32 or 64 */                                         \
-  X(128, 4, true, EPI_SPLIT, false, false, 64, 64) X(kTcBlockN, 3, true, EPI_SPLIT, false, false, 64, 64)      \
-  X(128, 6, false, EPI_SPLIT, false, false, 64, 64) X(kTcBlockN, 4, false, EPI_SPLIT, false, false, 64, 64)    \
-  X(128, 8, true, EPI_SPLIT, false, false, 32, 64) X(kTcBlockN, 6, true, EPI_SPLIT, false, false, 32, 64)      \
-  X(128, 12, false, EPI_SPLIT, false, false, 32, 64) X(kTcBlockN, 8, false, EPI_SPLIT, false, false, 32, 64)
+  X(128, 4, true, EPI_SPLIT, false, false, 64, 64, false) X(kTcBlockN, 3, true, EPI_SPLIT, false, false, 64, 64, false)      \
+  X(128, 6, false, EPI_SPLIT, false, false, 64, 64, false) X(kTcBlockN, 4, false, EPI_SPLIT, false, false, 64, 64, false)    \
+  X(128, 8, true, EPI_SPLIT, false, false, 32, 64, false) X(kTcBlockN, 6, true, EPI_SPLIT, false, false, 32, 64, false)      \
+  X(128, 12, false, EPI_SPLIT, false, false, 32, 64, false) X(kTcBlockN, 8, false, EPI_SPLIT, false, false, 32, 64, false) \
+  /* output rows that TMA cannot store */                                                                       \
+  X(128, 4, true, EPI_SPLIT, false, true, 64, 128, true) X(kTcBlockN, 3, true, EPI_SPLIT, false, true, 64, 128, true)    \
+  X(128, 4, true, EPI_SPLIT, false, false, 64, 128, true) X(kTcBlockN, 3, true, EPI_SPLIT, false, false, 64, 128, true)  \
+  X(128, 6, false, EPI_SPLIT, false, true, 64, 128, true) X(kTcBlockN, 4, false, EPI_SPLIT, false, true, 64, 128, true)  \
+  X(128, 6, false, EPI_SPLIT, false, false, 64, 128, true) X(kTcBlockN, 4, false, EPI_SPLIT, false, false, 64, 128, true)
 
 // Form choice.  Cluster flavour: f32 probabilities and 128-column tiles take the split
 // epilogue; 256-column f16 tiles take the relay when a CTA sees several tiles (its two groups
@@ -1175,7 +1240,13 @@ bool tc_stage_depth_legal(bool tiled, int bn, bool out_f32, int kd, int tm) {
 }
 
 TcVariant tc_choose_variant(bool tiled, int bn, bool out_f32, int batch, int num_rb, int num_kb, int cluster_n,
-                            int epilogue_mode, int pair_mode, int num_sms, int resident, int kd, int tm) {
+                            int epilogue_mode, int pair_mode, int num_sms, int resident, int kd, int tm, bool direct) {
+  if (direct) {
+    // split form, no CTA pairs, default tiles (as a relay, whose storing warps are fewer: 47 against 42 us for 24504 x 1021 x 64)
+    TcVariant v = tc_choose_variant(tiled, bn, out_f32, batch, num_rb, num_kb, cluster_n, kEpilogueSplit, 1, num_sms, 0);
+    v.direct = 1;
+    return v;
+  }
   if ((kd != kTcBlockK || tm != kTcBlockM) && tc_stage_depth_legal(tiled, bn, out_f32, kd, tm)) {
     // as many stages as keep the default's K depth in flight (more than its bytes, with 64-row tiles)
     const int st_cl = bn == 128 ? (kd == 32 ? 8 : (kd == 64 ? 4 : 2)) : (kd == 32 ? 6 : 3);
@@ -1201,8 +1272,8 @@ TcVariant tc_choose_variant(bool tiled, int bn, bool out_f32, int batch, int num
 }
 
 int tc_variant_smem_bytes(const TcVariant &v) {
-#define X(BN, ST, CL, EP, PA, O32, KD, TM) \
-  if (v.bn == BN && v.stages == ST && (v.cluster != 0) == CL && v.epi == EP && (v.pair != 0) == PA && (v.out32 != 0) == O32 && v.kd == KD && v.tm == TM) \
+#define X(BN, ST, CL, EP, PA, O32, KD, TM, DI) \
+  if (v.bn == BN && v.stages == ST && (v.cluster != 0) == CL && v.epi == EP && (v.pair != 0) == PA && (v.out32 != 0) == O32 && v.kd == KD && v.tm == TM && (v.direct != 0) == DI) \
     return SmemLayout<BN, ST, CL, EP, PA, O32, KD, TM>::kDynamic;
   WTC_TC_VARIANTS(X)
 #undef X
@@ -1214,9 +1285,9 @@ int tc_variant_threads(const TcVariant &v) { return kThreadsFor(v.epi); }
 namespace {
 cudaError_t launch_variant(const TcVariant &v, const CUtensorMap &tmA, const CUtensorMap &tmB, const CUtensorMap &tmO,
                            const TcParams &p, int cluster_n, int num_sms, cudaStream_t s, TcLaunchInfo *info) {
-#define X(BN, ST, CL, EP, PA, O32, KD, TM) \
-  if (v.bn == BN && v.stages == ST && (v.cluster != 0) == CL && v.epi == EP && (v.pair != 0) == PA && (v.out32 != 0) == O32 && v.kd == KD && v.tm == TM) \
-    return launch_impl<BN, ST, CL, EP, PA, O32, KD, TM>(tmA, tmB, tmO, p, cluster_n, num_sms, s, info);
+#define X(BN, ST, CL, EP, PA, O32, KD, TM, DI) \
+  if (v.bn == BN && v.stages == ST && (v.cluster != 0) == CL && v.epi == EP && (v.pair != 0) == PA && (v.out32 != 0) == O32 && v.kd == KD && v.tm == TM && (v.direct != 0) == DI) \
+    return launch_impl<BN, ST, CL, EP, PA, O32, KD, TM, DI>(tmA, tmB, tmO, p, cluster_n, num_sms, s, info);
   WTC_TC_VARIANTS(X)
 #undef X
   return cudaErrorInvalidConfiguration;
@@ -1230,7 +1301,8 @@ cudaError_t launch_fused_cluster(const CUtensorMap &tmA, const CUtensorMap &tmB,
   // the single-tile form is tried whenever one tile per CTA is possible at all; it declines
   // (before launching) when the clusters do not all fit the chip at once, and the split form runs
   TcVariant v = tc_choose_variant(false, bn, p.out_f32 != 0, p.batch, p.num_rb, p.num_kb, cluster_n, p.epilogue_mode, p.pair_mode,
-                                  num_sms, /*resident=*/1 << 30, p.stage_k ? p.stage_k : kTcBlockK, p.tile_rows ? p.tile_rows : kTcBlockM);
+                                  num_sms, /*resident=*/1 << 30, p.stage_k ? p.stage_k : kTcBlockK, p.tile_rows ? p.tile_rows : kTcBlockM,
+                                  p.direct_out != 0);
   if (v.epi == EPI_SINGLE) {
     const cudaError_t e = launch_variant(v, tmA, tmB, tmO, p, cluster_n, num_sms, s, info);
     if (e != cudaErrorNotSupported) return e;
@@ -1242,7 +1314,7 @@ cudaError_t launch_fused_cluster(const CUtensorMap &tmA, const CUtensorMap &tmB,
 cudaError_t launch_tiled_partial(const CUtensorMap &tmA, const CUtensorMap &tmB, const CUtensorMap &tmO,
                                  const TcParams &p, int bn, int num_sms, cudaStream_t s, TcLaunchInfo *info) {
   const TcVariant v = tc_choose_variant(true, bn, p.out_f32 != 0, p.batch, p.num_rb, p.num_kb, 1, p.epilogue_mode, p.pair_mode, num_sms, 0,
-                                        p.stage_k ? p.stage_k : kTcBlockK, p.tile_rows ? p.tile_rows : kTcBlockM);
+                                        p.stage_k ? p.stage_k : kTcBlockK, p.tile_rows ? p.tile_rows : kTcBlockM, p.direct_out != 0);
   return launch_variant(v, tmA, tmB, tmO, p, 1, num_sms, s, info);
 }
 

@@ -104,8 +104,27 @@ rescale_rows_kernel(void *__restrict__ out_v, int out_f32, int N, int64_t ld_out
       o4[j] = x;
     }
   } else {
-    for (int j = c0 + threadIdx.x; j < c1; j += blockDim.x)
+    // rows that start or end anywhere: element by element up to the first 16-byte boundary and behind
+    // the last whole vector; a vector may lie across two tiles
+    const int head = min(static_cast<int>((8 - ((reinterpret_cast<uintptr_t>(orow + c0) >> 1) & 7)) & 7), c1 - c0);
+    const int v0 = c0 + head, v1 = v0 + ((c1 - v0) & ~7);
+    for (int j = v0 + threadIdx.x * 8; j < v1; j += blockDim.x * 8) {
+      const int t0 = j / BN, split = (t0 + 1) * BN - j;      // elements from `split` on belong to the next tile
+      const float f0 = factor[t0], f1 = split < 8 ? factor[t0 + 1] : f0;
+      uint4 x = *reinterpret_cast<uint4 *>(orow + j);
+      __half2 *h = reinterpret_cast<__half2 *>(&x);
+#pragma unroll
+      for (int i = 0; i < 4; ++i) {
+        const float2 t = __half22float2(h[i]);
+        h[i] = __floats2half2_rn(t.x * (2 * i < split ? f0 : f1), t.y * (2 * i + 1 < split ? f0 : f1));
+      }
+      *reinterpret_cast<uint4 *>(orow + j) = x;
+    }
+    const int ends = head + (c1 - v1);
+    if (static_cast<int>(threadIdx.x) < ends) {
+      const int j = static_cast<int>(threadIdx.x) < head ? c0 + static_cast<int>(threadIdx.x) : v1 + static_cast<int>(threadIdx.x) - head;
       orow[j] = __float2half_rn(__half2float(orow[j]) * factor[j / BN]);
+    }
   }
 }
 
@@ -156,69 +175,86 @@ cudaError_t launch_rescale_rows(void *out, int out_f32, int64_t rows, int N, int
                             global_stats, num_parts, rows, chunk);
 }
 
-// ---- f32 -> f16 rounding of both operands (the chain that truncates its f32 arguments) --------
+// ---- operand copies -----------------------------------------------------------------------------
+// For the chain that truncates its f32 arguments to f16, and for f16 operands whose rows TMA cannot
+// read (strides that are no multiple of 16 bytes).
 namespace {
-struct RoundJob {
-  const float *src; __half *dst;
-  int64_t rows, cols, ld, batch_stride, work;   // work: quads (vec) or elements
-  int vec;
+struct CopyJob {
+  const void *src; __half *dst;
+  int64_t ld, batch_stride;
+  int64_t rows, cols, per_row, work;     // rows of one batch; work = units of eight destination columns, per_row of them a row
+  int vec;                               // whole units can be read with 16-byte loads
 };
 
-__device__ __forceinline__ void round_one(const RoundJob &j, int64_t q) {
-  if (j.vec) {
-    const int64_t per_row = j.cols >> 2;
-    const int64_t row = q / per_row, c = (q - row * per_row) << 2;
-    const int64_t b = row / j.rows, r = row - b * j.rows;
-    const float4 v = *reinterpret_cast<const float4 *>(j.src + b * j.batch_stride + r * j.ld + c);
-    const __half2 lo = __floats2half2_rn(v.x, v.y), hi = __floats2half2_rn(v.z, v.w);
-    uint2 o;
-    o.x = *reinterpret_cast<const uint32_t *>(&lo);
-    o.y = *reinterpret_cast<const uint32_t *>(&hi);
-    *reinterpret_cast<uint2 *>(j.dst + row * j.cols + c) = o;
+// I: what units are counted in (32 bits unless there are more than 2^32 of them: its divisions are several times shorter)
+template <bool F32, typename I>
+__device__ __forceinline__ void copy_unit(const CopyJob &j, I u) {
+  const I row = u / static_cast<I>(j.per_row);
+  const int64_t c = static_cast<int64_t>(u - row * static_cast<I>(j.per_row)) * 8;
+  const I b = row / static_cast<I>(j.rows), r = row - b * static_cast<I>(j.rows);
+  const int64_t at = static_cast<int64_t>(b) * j.batch_stride + static_cast<int64_t>(r) * j.ld + c;
+  uint32_t w[4];
+  if (F32) {
+    const float *src = static_cast<const float *>(j.src) + at;
+    float v[8];
+    if (j.vec && c + 8 <= j.cols) {
+      const float4 lo = *reinterpret_cast<const float4 *>(src), hi = *reinterpret_cast<const float4 *>(src + 4);
+      v[0] = lo.x; v[1] = lo.y; v[2] = lo.z; v[3] = lo.w;
+      v[4] = hi.x; v[5] = hi.y; v[6] = hi.z; v[7] = hi.w;
+    } else {
+#pragma unroll
+      for (int e = 0; e < 8; ++e) v[e] = c + e < j.cols ? src[e] : 0.f;
+    }
+#pragma unroll
+    for (int e = 0; e < 4; ++e) w[e] = pack_f16x2(v[2 * e], v[2 * e + 1]);
   } else {
-    const int64_t row = q / j.cols, c = q - row * j.cols;
-    const int64_t b = row / j.rows, r = row - b * j.rows;
-    j.dst[q] = __float2half_rn(j.src[b * j.batch_stride + r * j.ld + c]);
+    const uint16_t *src = static_cast<const uint16_t *>(j.src) + at;
+    if (j.vec && c + 8 <= j.cols) {
+      const uint4 o = *reinterpret_cast<const uint4 *>(src);
+      w[0] = o.x; w[1] = o.y; w[2] = o.z; w[3] = o.w;
+    } else {
+      uint32_t h[8];
+#pragma unroll
+      for (int e = 0; e < 8; ++e) h[e] = c + e < j.cols ? src[e] : 0u;
+#pragma unroll
+      for (int e = 0; e < 4; ++e) w[e] = h[2 * e] | h[2 * e + 1] << 16;
+    }
   }
+  *reinterpret_cast<uint4 *>(j.dst + static_cast<int64_t>(u) * 8) = make_uint4(w[0], w[1], w[2], w[3]);
 }
 
-// One launch rounds A and B: one thread per four consecutive columns of a row (or per element
-// when the rows are not 16-byte friendly), the work items of A first, then B's.  Launched with
-// programmatic stream serialisation: the chain's kernel behind it starts its set-up as soon as
-// these CTAs are resident, and waits for them to finish before its first load.
-__global__ void round_to_f16_kernel(const RoundJob a, const RoundJob b) {
+// One launch copies A and B: one thread per eight destination columns, A's units first, then B's.
+// Launched with programmatic stream serialisation: the chain's kernel behind it starts its set-up
+// as soon as these CTAs are resident, and waits for them to finish before its first load.
+template <bool F32, typename I>
+__global__ void __launch_bounds__(256) copy_operands_kernel(const CopyJob a, const CopyJob b) {
   grid_dependency_wait();                    // the operands may be the previous kernel's output
   grid_launch_dependents();
-  const int64_t total = a.work + b.work;
-  for (int64_t q = blockIdx.x * static_cast<int64_t>(blockDim.x) + threadIdx.x; q < total;
-       q += static_cast<int64_t>(gridDim.x) * blockDim.x) {
-    if (q < a.work) round_one(a, q);
-    else round_one(b, q - a.work);
-  }
+  const int64_t u = blockIdx.x * int64_t{256} + threadIdx.x;
+  if (u < a.work) copy_unit<F32, I>(a, static_cast<I>(u));
+  else if (u < a.work + b.work) copy_unit<F32, I>(b, static_cast<I>(u - a.work));
 }
 
-RoundJob make_job(const float *src, void *dst, int batch, int64_t rows, int64_t cols, int64_t ld, int64_t batch_stride) {
-  RoundJob j;
-  j.src = src; j.dst = static_cast<__half *>(dst);
-  j.rows = rows; j.cols = cols; j.ld = ld; j.batch_stride = batch_stride;
-  const int64_t total = static_cast<int64_t>(batch) * rows * cols;
-  j.vec = (cols % 4 == 0) && (ld % 4 == 0) && (batch_stride % 4 == 0) && ((reinterpret_cast<uintptr_t>(src) & 15) == 0) &&
-          ((reinterpret_cast<uintptr_t>(dst) & 7) == 0);
-  j.work = j.vec ? total / 4 : total;
+CopyJob make_job(const OperandCopy &c, bool f32) {
+  CopyJob j{};
+  if (!c.dst) return j;
+  j.src = c.src; j.dst = static_cast<__half *>(c.dst);
+  j.ld = c.ld; j.batch_stride = c.batch_stride;
+  j.rows = c.rows; j.cols = c.cols; j.per_row = c.ld_dst / 8;
+  j.work = c.batch * c.rows * j.per_row;
+  const int per16 = f32 ? 4 : 8;
+  j.vec = c.ld % per16 == 0 && (c.batch == 1 || c.batch_stride % per16 == 0) && (reinterpret_cast<uintptr_t>(c.src) & 15) == 0;
   return j;
 }
 } // namespace
 
-cudaError_t launch_round_to_f16(const float *A, void *dstA, int batchA, int64_t rowsA, int64_t colsA, int64_t ldA, int64_t strideA,
-                                const float *B, void *dstB, int batchB, int64_t rowsB, int64_t colsB, int64_t ldB, int64_t strideB,
-                                cudaStream_t s) {
-  const RoundJob a = make_job(A, dstA, batchA, rowsA, colsA, ldA, strideA);
-  const RoundJob b = make_job(B, dstB, batchB, rowsB, colsB, ldB, strideB);
-  const int64_t work = a.work + b.work;
+cudaError_t launch_copy_operands(const OperandCopy &a, const OperandCopy &b, bool src_f32, cudaStream_t s) {
+  const CopyJob ja = make_job(a, src_f32), jb = make_job(b, src_f32);
+  const int64_t work = ja.work + jb.work;
   if (work == 0) return cudaSuccess;
-  const int64_t blocks = (work + 255) / 256;
+  if ((work + 255) / 256 > 0x7fffffff) return cudaErrorInvalidConfiguration;
   cudaLaunchConfig_t cfg = {};
-  cfg.gridDim = dim3(static_cast<unsigned>(blocks < 148 * 16 ? blocks : 148 * 16), 1, 1);
+  cfg.gridDim = dim3(static_cast<unsigned>((work + 255) / 256), 1, 1);
   cfg.blockDim = dim3(256, 1, 1);
   cfg.stream = s;
   cudaLaunchAttribute attr[1];
@@ -226,7 +262,9 @@ cudaError_t launch_round_to_f16(const float *A, void *dstA, int batchA, int64_t 
   attr[0].val.programmaticStreamSerializationAllowed = 1;
   cfg.attrs = attr;
   cfg.numAttrs = 1;
-  return cudaLaunchKernelEx(&cfg, round_to_f16_kernel, a, b);
+  const bool wide = ja.work >= (int64_t{1} << 32) || jb.work >= (int64_t{1} << 32);
+  if (src_f32) return wide ? cudaLaunchKernelEx(&cfg, copy_operands_kernel<true, uint64_t>, ja, jb) : cudaLaunchKernelEx(&cfg, copy_operands_kernel<true, uint32_t>, ja, jb);
+  return wide ? cudaLaunchKernelEx(&cfg, copy_operands_kernel<false, uint64_t>, ja, jb) : cudaLaunchKernelEx(&cfg, copy_operands_kernel<false, uint32_t>, ja, jb);
 }
 
 } // namespace wtc

@@ -554,6 +554,8 @@ cudaError_t launch_tiles(const void *A, const void *B, void *Out, const SimtPara
 
 } // namespace
 
+bool simt_fused_takes(const SimtParams &p) { return pick_rows(p, kRowLimit) != 0; }
+
 int simt_fused_launches(const SimtParams &p) {
   return use_tiles(p, pick_rows(p, kRowLimit)) && p.N > 8 * kTileChoices[pick_tile(p)].bn ? 2 : 1;
 }

@@ -34,6 +34,10 @@ struct TcParams {
   float c2;        // scale * log2(e)
   float2 *tile_stats;    // tiled mode: [batch*M][num_nb] (max in log2 domain, sum of 2^(v-max))
   int *status;     // device status word (0 = ok)
+  // rows of the output that TMA cannot store (strides that are no multiple of 16 bytes): written from the staging tiles
+  int direct_out;
+  void *out;
+  int64_t ldo, o_batch_stride;
 #ifdef WTC_BRINGUP
   long long *timeline;   // optional [grid][48] stamps of each CTA's first tile: %globaltimer ns in 0..23, clock64 in 24..47
 #endif
@@ -49,12 +53,13 @@ struct TcVariant {
   int bn, stages, cluster, epi, pair, out32;
   int kd;    // K depth of one pipeline stage: 64, or the schedule's tileK when it is 32 or 128 and legal
   int tm;    // rows of a tile: 128, or the schedule's tileM when it is 64 and legal
+  int direct = 0;   // the output rows are written by the epilogue's threads instead of TMA stores
 };
 // The variant the launchers below take for a call, worked out without a device: `resident` is how
 // many clusters of `cluster_n` CTAs the chip holds at once (the launchers ask the runtime; a plan
 // made without a device uses the figures measured on a 148-SM part).
 TcVariant tc_choose_variant(bool tiled, int bn, bool out_f32, int batch, int num_rb, int num_kb, int cluster_n,
-                            int epilogue_mode, int pair_mode, int num_sms, int resident, int kd = 64, int tm = 128);
+                            int epilogue_mode, int pair_mode, int num_sms, int resident, int kd = 64, int tm = 128, bool direct = false);
 // Whether this stage depth and tile height have a kernel for this flavour, column tile and output type.
 bool tc_stage_depth_legal(bool tiled, int bn, bool out_f32, int kd, int tm = 128);
 // Dynamic shared memory and threads per CTA of a variant (0 if it is not instantiated).
@@ -81,11 +86,14 @@ cudaError_t launch_rescale_rows(void *out, int out_f32, int64_t rows, int N, int
                                 const float2 *tile_stats, const float2 *global_stats, int num_parts,
                                 cudaStream_t s);
 
-// For both operands in one launch: dst[b][r][c] (dense f16: row stride cols, batch stride rows * cols)
-// = round-to-nearest-even of src[b * batch_stride + r * ld + c] (f32).
-cudaError_t launch_round_to_f16(const float *A, void *dstA, int batchA, int64_t rowsA, int64_t colsA, int64_t ldA, int64_t strideA,
-                                const float *B, void *dstB, int batchB, int64_t rowsB, int64_t colsB, int64_t ldB, int64_t strideB,
-                                cudaStream_t s);
+// Copies of the operands that the tensor-core kernels can read, both in one launch: dst[b][r][0..ld_dst) (dense f16,
+// ld_dst a multiple of 8) = src[b * batch_stride + r * ld + c], rounded to nearest even when the source is f32, zeros
+// from column `cols` on.  An operand whose `dst` is null is left alone.
+struct OperandCopy {
+  const void *src; void *dst;
+  int64_t batch, rows, cols, ld, batch_stride, ld_dst;
+};
+cudaError_t launch_copy_operands(const OperandCopy &a, const OperandCopy &b, bool src_f32, cudaStream_t s);
 
 // The four softmax passes of the unfused baseline on logits C32[rows, N] already in global
 // memory: row max -> exp -> row sum -> divide (intermediates E[rows, N], mx[rows], sum[rows]).
@@ -108,6 +116,7 @@ struct SimtParams {
   float scale;
 };
 cudaError_t launch_simt_fused(const void *A, const void *B, void *Out, const SimtParams &p, cudaStream_t s);
+bool simt_fused_takes(const SimtParams &p);     // whether a row is short enough for the SIMT path
 int simt_fused_launches(const SimtParams &p);
 // Unfused five-kernel pipeline: matmul -> row max -> exp -> row sum -> divide,
 // with C32[M,N], max[M], E[M,N], sum[M] in global memory (workspace).

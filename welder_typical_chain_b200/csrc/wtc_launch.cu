@@ -45,13 +45,13 @@ const int g_use_pdl = [] { const char *e = getenv("WTC_NO_PDL"); return (e && e[
 
 // registers / spills / stack of every instance of the tensor-core kernel template, from the
 // `ptxas -v` report of this build (generated beside the objects)
-struct KernelFacts { int bn, stages, cluster, epi, pair, out32, kd, tm, registers, spill_store, spill_load, stack; };
+struct KernelFacts { int bn, stages, cluster, epi, pair, out32, kd, tm, direct, registers, spill_store, spill_load, stack; };
 const KernelFacts kKernelFacts[] = {
 #include "build/kernel_facts.inc"
 };
 const KernelFacts *facts_of(const wtc::TcVariant &v) {
   for (const KernelFacts &f : kKernelFacts)
-    if (f.bn == v.bn && f.stages == v.stages && f.cluster == (v.cluster != 0) && f.epi == v.epi && f.pair == (v.pair != 0) && f.out32 == (v.out32 != 0) && f.kd == v.kd && f.tm == v.tm)
+    if (f.bn == v.bn && f.stages == v.stages && f.cluster == (v.cluster != 0) && f.epi == v.epi && f.pair == (v.pair != 0) && f.out32 == (v.out32 != 0) && f.kd == v.kd && f.tm == v.tm && f.direct == (v.direct != 0))
       return &f;
   return nullptr;
 }
@@ -65,6 +65,11 @@ struct Resolved {
   int num_rb, num_nb, num_kb;
   bool b_batched;
   bool tc_ok;
+  // f16 chains with rows TMA cannot take (strides that are no multiple of 16 bytes): operands read from padded
+  // copies in the workspace (copy_a / copy_b: their bytes, 0 = read in place), output rows written by the epilogue
+  bool ragged;
+  size_t copy_a, copy_b;
+  bool direct_out;
   // WTC_FLAG_MATMUL_F16: f32 operands are first rounded to dense f16 copies at the head of the
   // workspace, then `inner` (the same chain on f16 operands) runs on the copies
   bool trunc = false;
@@ -75,6 +80,11 @@ struct Resolved {
 size_t align256(size_t v) { return (v + 255) & ~static_cast<size_t>(255); }
 
 bool mult8(int64_t v) { return (v & 7) == 0; }
+int64_t round8(int64_t v) { return (v + 7) & ~static_cast<int64_t>(7); }
+int64_t round64(int64_t v) { return (v + 63) & ~static_cast<int64_t>(63); }
+// Multiply-adds from which a ragged f16 chain goes to the tensor cores: below, the SIMT row kernel's one launch is faster
+// than an operand copy and a chain (500 x 333 x 64: 9.2 against 10.0 us; 1000 x 1001 x 16: 12.3 against 10.5 us).
+constexpr double kRaggedMinWork = 12 << 20;
 
 wtc::SimtParams simt_params(const Resolved &r) {
   wtc::SimtParams s;
@@ -118,8 +128,8 @@ int resolve(const wtc_chain_desc *in, Resolved &r) {
     wtc_chain_desc inner = d;
     inner.in_dtype = WTC_F16;
     inner.flags &= ~WTC_FLAG_MATMUL_F16;
-    inner.lda = d.K; inner.a_batch_stride = d.M * d.K;
-    inner.ldb = d.N; inner.b_batch_stride = r.b_batched ? d.K * d.N : -1;
+    inner.lda = round8(d.K); inner.a_batch_stride = d.M * inner.lda;     // rows TMA can read, whatever K and N
+    inner.ldb = round8(d.N); inner.b_batch_stride = r.b_batched ? d.K * inner.ldb : -1;
     Resolved ri;
     int rc = resolve(&inner, ri);
     if (rc) return rc;
@@ -131,8 +141,8 @@ int resolve(const wtc_chain_desc *in, Resolved &r) {
     r.inner = inner;
     r.trunc = true;
     r.tc_ok = false;          // the sharded and static-scratch entry points take f16 operands only
-    r.stage_a = align256(static_cast<size_t>(d.batch) * d.M * d.K * 2);
-    r.stage_b = align256(static_cast<size_t>(bb ? d.batch : 1) * d.K * d.N * 2);
+    r.stage_a = align256(static_cast<size_t>(d.batch) * d.M * inner.lda * 2);
+    r.stage_b = align256(static_cast<size_t>(bb ? d.batch : 1) * d.K * inner.ldb * 2);
     r.plan.workspace_bytes += r.stage_a + r.stage_b;
     r.plan.launches += 1;     // one launch rounds both operands
     return WTC_OK;
@@ -183,6 +193,24 @@ int resolve(const wtc_chain_desc *in, Resolved &r) {
                         mult8(d.a_batch_stride) && mult8(d.b_batch_stride) && mult8(d.o_batch_stride) &&
                         static_cast<int64_t>(d.batch) * r.num_rb * r.num_nb < 0x7fffffff;
   r.tc_ok = tc_shape && !(d.flags & WTC_FLAG_FORCE_SIMT) && d.variant == WTC_VARIANT_FUSED;
+  // ... and the shapes that become such a chain with padded copies of the operands and rows the epilogue writes itself.
+  // Only what the SIMT kernel takes too (its row of logits in shared memory), since a call without the workspace, or with
+  // pointers off their 16-byte boundaries, runs there.
+  const bool tiled_row = r.num_nb > 8 || (d.flags & WTC_FLAG_FORCE_TILED);
+  r.copy_a = r.copy_b = 0;
+  r.direct_out = false;
+  r.ragged = !tc_shape && d.in_dtype == WTC_F16 && d.M > 0 && d.N > 0 && d.K > 0 && d.variant == WTC_VARIANT_FUSED &&
+             !(d.flags & WTC_FLAG_FORCE_SIMT) && static_cast<double>(d.batch) * d.M * d.N * d.K >= kRaggedMinWork &&
+             wtc::simt_fused_takes(simt_params(r)) && static_cast<int64_t>(d.batch) * r.num_rb * r.num_nb < 0x7fffffff &&
+             !(tiled_row && d.batch > 1 && d.o_batch_stride != d.M * d.ldo);
+  if (r.ragged) {
+    r.kd = wtc::kTcBlockK; r.tm = wtc::kTcBlockM;           // these kernels exist for the default tiles only
+    r.num_rb = static_cast<int>((d.M + wtc::kTcBlockM - 1) / wtc::kTcBlockM);
+    r.num_kb = static_cast<int>((d.K + r.kd - 1) / r.kd);
+    if (!mult8(d.K) || !mult8(d.lda) || !mult8(d.a_batch_stride)) r.copy_a = align256(static_cast<size_t>(d.batch) * d.M * round8(d.K) * 2);
+    if (!mult8(d.ldb) || !mult8(d.b_batch_stride)) r.copy_b = align256(static_cast<size_t>(r.b_batched ? d.batch : 1) * d.K * round64(d.N) * 2);
+    r.direct_out = !mult8(d.N) || !mult8(d.ldo) || !mult8(d.o_batch_stride);      // (a TMA store fills the last 16 bytes of a row)
+  }
 
   if (d.variant == WTC_VARIANT_BASELINE) {
     // five kernels with C32[rows,N], E[rows,N], max[rows], sum[rows] in global memory.  For f16
@@ -202,7 +230,7 @@ int resolve(const wtc_chain_desc *in, Resolved &r) {
       p.threads = 256;
       p.tile_m = 8; p.tile_n = static_cast<int32_t>(d.N); p.tile_k = 64;
     }
-  } else if (r.tc_ok) {
+  } else if (r.tc_ok || r.ragged) {
     p.tile_m = r.tm; p.tile_n = r.bn; p.tile_k = r.kd;
     p.tmem_columns = 2 * r.bn;
     // variant, threads, stages as the launchers choose them on a 148-SM part (the plan is made
@@ -214,7 +242,7 @@ int resolve(const wtc_chain_desc *in, Resolved &r) {
     const bool cluster = r.num_nb <= 8 && !(d.flags & WTC_FLAG_FORCE_TILED);
     const wtc::TcVariant v = wtc::tc_choose_variant(!cluster, r.bn, d.out_dtype == WTC_F32, d.batch, r.num_rb, r.num_kb,
                                                     cluster ? r.num_nb : 1, epi_mode, pair_mode, 148,
-                                                    cluster ? kResidentClusters[r.num_nb] : 0, r.kd, r.tm);
+                                                    cluster ? kResidentClusters[r.num_nb] : 0, r.kd, r.tm, r.direct_out);
     p.threads = wtc::tc_variant_threads(v);
     p.stages = v.stages;
     p.smem_bytes = wtc::tc_variant_smem_bytes(v);
@@ -227,6 +255,10 @@ int resolve(const wtc_chain_desc *in, Resolved &r) {
       p.kernel = WTC_KERNEL_TC_TILED;
       p.launches = 2;
       p.workspace_bytes = static_cast<size_t>(d.batch) * d.M * r.num_nb * sizeof(float2);
+    }
+    if (r.copy_a || r.copy_b) {
+      p.launches += 1;        // one launch copies both operands
+      p.workspace_bytes += r.copy_a + r.copy_b;
     }
   } else {
     p.kernel = WTC_KERNEL_SIMT_FUSED;
@@ -315,7 +347,11 @@ int get_map(const void *ptr, uint64_t d0, uint64_t d1, uint64_t d2, uint64_t s1_
 // [batch][N/64][K][64]: one copy then brings `blocks` 64-column blocks of a K block, each laid
 // out as the tensor core wants it (one stage's k-rows x 128 bytes); otherwise one copy per 64 columns.
 int get_map_b(const void *B, const Resolved &r, int blocks, CUtensorMap *out, int *b_blocks) {
-  const wtc_chain_desc &d = r.d;
+  wtc_chain_desc d = r.d;
+  if (r.copy_b) {                                   // the padded copy: rows of whole 64-column blocks, zeros behind column N
+    d.N = d.ldb = round64(d.N);
+    d.b_batch_stride = d.K * d.ldb;
+  }
   const uint64_t nbatch = r.b_batched ? d.batch : 1;
   const uint64_t bstride = (r.b_batched ? d.b_batch_stride : d.K * d.ldb) * 2;
   if (d.N % 64 == 0) {
@@ -380,9 +416,9 @@ int launch_resolved(Resolved &r, const void *A, const void *B, void *Out, void *
       return fail(WTC_E_WORKSPACE, "rounding the f32 operands to f16 needs %zu workspace bytes, got %zu", r.plan.workspace_bytes, ws_bytes);
     if ((reinterpret_cast<uintptr_t>(ws) & 15) != 0) return fail(WTC_E_ARG, "workspace must be 16-byte aligned");
     unsigned char *base = static_cast<unsigned char *>(ws);
-    const cudaError_t e = wtc::launch_round_to_f16(static_cast<const float *>(A), base, d.batch, d.M, d.K, d.lda, d.a_batch_stride,
-                                                   static_cast<const float *>(B), base + r.stage_a, r.b_batched ? d.batch : 1, d.K, d.N, d.ldb,
-                                                   r.b_batched ? d.b_batch_stride : 0, s);
+    const wtc::OperandCopy ca{A, base, d.batch, d.M, d.K, d.lda, d.a_batch_stride, r.inner.lda};
+    const wtc::OperandCopy cb{B, base + r.stage_a, r.b_batched ? d.batch : 1, d.K, d.N, d.ldb, r.b_batched ? d.b_batch_stride : 0, r.inner.ldb};
+    const cudaError_t e = wtc::launch_copy_operands(ca, cb, true, s);
     if (e != cudaSuccess) return cuda_fail(e, "operand rounding launch");
     Resolved ri;
     int rc = resolve(&r.inner, ri);
@@ -434,23 +470,43 @@ int launch_resolved(Resolved &r, const void *A, const void *B, void *Out, void *
     return e == cudaSuccess ? WTC_OK : cuda_fail(e, "unfused tensor-core pipeline launch");
   }
 
-  const bool ptr_ok = aligned16(A) && aligned16(B) && aligned16(Out);
+  const bool ws_ok = !r.ragged || r.plan.workspace_bytes == 0 || (ws && ws_bytes >= r.plan.workspace_bytes && aligned16(ws));
+  const bool ptr_ok = (r.copy_a || aligned16(A)) && (r.copy_b || aligned16(B)) && (r.direct_out || aligned16(Out)) && ws_ok;
   bool tiled = r.plan.kernel == WTC_KERNEL_TC_TILED || (mode == 1 && r.tc_ok);
   if ((r.plan.kernel == WTC_KERNEL_TC_CLUSTER || tiled) && ptr_ok) {
     const int sms = num_sms();
     if (sms <= 0) return fail(WTC_E_CUDA, "no usable CUDA device");
+    int64_t lda = d.lda, a_batch_stride = d.a_batch_stride;
+    if (r.copy_a || r.copy_b) {
+      unsigned char *base = static_cast<unsigned char *>(ws);
+      wtc::OperandCopy ca{}, cb{};
+      if (r.copy_a) {
+        ca = wtc::OperandCopy{A, base, d.batch, d.M, d.K, d.lda, d.a_batch_stride, round8(d.K)};
+        A = base;
+        lda = round8(d.K); a_batch_stride = d.M * lda;
+      }
+      if (r.copy_b) {
+        cb = wtc::OperandCopy{B, base + r.copy_a, r.b_batched ? d.batch : 1, d.K, d.N, d.ldb, r.b_batched ? d.b_batch_stride : 0, round64(d.N)};
+        B = base + r.copy_a;
+      }
+      const cudaError_t e = wtc::launch_copy_operands(ca, cb, false, s);
+      if (e != cudaSuccess) return cuda_fail(e, "operand copy launch");
+      ws = base + r.copy_a + r.copy_b;
+      ws_bytes -= r.copy_a + r.copy_b;
+    }
     CUtensorMap tmA, tmB, tmO;
     // A's box is one swizzle span wide at most: 64 columns (a 128-deep stage takes two), or 32 with the 64-byte swizzle
-    int rc = get_map(A, d.K, d.M, d.batch, d.lda * 2, d.a_batch_stride * 2, r.kd < 64 ? r.kd : 64, r.tm, &tmA, false, 0, 0, 1, r.kd == 32);
+    int rc = get_map(A, d.K, d.M, d.batch, lda * 2, a_batch_stride * 2, r.kd < 64 ? r.kd : 64, r.tm, &tmA, false, 0, 0, 1, r.kd == 32);
     if (rc) return rc;
     // (a CTA pair loads half of the tile's columns per CTA: the variant decides the box)
     const int pm = (d.flags & WTC_FLAG_NO_PAIR) ? 1 : ((d.flags & WTC_FLAG_PAIR) ? 2 : 0);
-    const wtc::TcVariant v = wtc::tc_choose_variant(tiled, r.bn, d.out_dtype == WTC_F32, d.batch, r.num_rb, r.num_kb, tiled ? 1 : r.num_nb, 0, pm, sms, 0, r.kd, r.tm);
+    const wtc::TcVariant v = wtc::tc_choose_variant(tiled, r.bn, d.out_dtype == WTC_F32, d.batch, r.num_rb, r.num_kb, tiled ? 1 : r.num_nb, 0, pm, sms, 0, r.kd, r.tm, r.direct_out);
     int b_blocks = 0;
     rc = get_map_b(B, r, v.pair ? r.bn / 128 : r.bn / 64, &tmB, &b_blocks);
     if (rc) return rc;
     const bool out32 = d.out_dtype == WTC_F32;
-    rc = out32 ? get_map(Out, d.N, d.M, d.batch, d.ldo * 4, d.o_batch_stride * 4, 32, 32, &tmO, true)
+    if (r.direct_out) tmO = tmA;                    // only prefetched
+    else rc = out32 ? get_map(Out, d.N, d.M, d.batch, d.ldo * 4, d.o_batch_stride * 4, 32, 32, &tmO, true)
                : get_map(Out, d.N, d.M, d.batch, d.ldo * 2, d.o_batch_stride * 2, 64, r.tm / 4, &tmO);   // a warp stores its quarter of the tile's rows
     if (rc) return rc;
 
@@ -468,8 +524,11 @@ int launch_resolved(Resolved &r, const void *A, const void *B, void *Out, void *
     p.timeline = g_timeline ? g_timeline + static_cast<size_t>(g_timeline_launch++ % 4) * 148 * 48 : nullptr;
 #endif
     p.use_pdl = g_use_pdl;
-    p.operands_ready = (d.flags & WTC_FLAG_OPERANDS_READY) ? 1 : 0;
+    p.operands_ready = (d.flags & WTC_FLAG_OPERANDS_READY) && !r.copy_a && !r.copy_b ? 1 : 0;   // (the copies are earlier work on the stream)
     p.out_f32 = out32;
+    p.direct_out = r.direct_out;
+    p.out = Out;
+    p.ldo = d.ldo; p.o_batch_stride = d.o_batch_stride;
     p.stage_k = r.kd;
     p.tile_rows = r.tm;
     p.pair_mode = (d.flags & WTC_FLAG_NO_PAIR) ? 1 : ((d.flags & WTC_FLAG_PAIR) ? 2 : 0);
