@@ -49,6 +49,9 @@ class ChainDesc(C.Structure):
     ]
 
 
+_CHAIN_DESC_SIZE = C.sizeof(ChainDesc)
+
+
 class RowChainDesc(C.Structure):
     _fields_ = [
         ("struct_size", C.c_int32), ("kind", C.c_int32), ("rows", C.c_int64), ("N", C.c_int64),
@@ -57,6 +60,7 @@ class RowChainDesc(C.Structure):
     ]
 
 
+_ROW_CHAIN_DESC_SIZE = C.sizeof(RowChainDesc)
 ROW_SOFTMAX, ROW_VARIANCE = 0, 1
 
 
@@ -111,18 +115,9 @@ def make_desc(batch: int, M: int, N: int, K: int, in_dtype: int = F16, out_dtype
               acc_dtype: int = F32, scale: float = 1.0, shared_b: bool = False, variant: int = VARIANT_FUSED,
               flags: int = 0, tile_m: int = 0, tile_n: int = 0, tile_k: int = 0,
               lda: int = 0, ldb: int = 0, ldo: int = 0) -> ChainDesc:
-    d = ChainDesc()
-    d.struct_size = C.sizeof(ChainDesc)
-    d.batch, d.M, d.N, d.K = batch, M, N, K
-    d.lda, d.ldb, d.ldo = lda, ldb, ldo
-    d.a_batch_stride = 0
-    d.b_batch_stride = -1 if shared_b else 0
-    d.o_batch_stride = 0
-    d.in_dtype, d.out_dtype, d.acc_dtype = in_dtype, out_dtype, acc_dtype
-    d.scale = scale
-    d.tile_m, d.tile_n, d.tile_k = tile_m, tile_n, tile_k
-    d.variant, d.flags = variant, flags
-    return d
+    # all fields in one construction, in the order of _fields_ (setting them one by one costs several times as much)
+    return ChainDesc(_CHAIN_DESC_SIZE, batch, M, N, K, lda, ldb, ldo, 0, -1 if shared_b else 0, 0, in_dtype, out_dtype, acc_dtype, scale,
+                     tile_m, tile_n, tile_k, variant, flags)
 
 
 def plan_query(desc: ChainDesc) -> PlanInfo:
@@ -139,34 +134,43 @@ def workspace_bytes(desc: ChainDesc) -> int:
 
 # ------------------------------------------------------------------ torch side
 
+_TORCH = None
+_CODE_OF: dict = {}
+
+
 def _torch():
-    import torch
-    return torch
+    global _TORCH
+    if _TORCH is None:
+        import torch
+        _CODE_OF.update({torch.float16: F16, torch.float32: F32})
+        _TORCH = torch
+    return _TORCH
 
 
 def _dt(t) -> int:
-    torch = _torch()
-    if t.dtype == torch.float16:
-        return F16
-    if t.dtype == torch.float32:
-        return F32
-    raise TypeError(f"unsupported dtype {t.dtype}")
+    _torch()
+    code = _CODE_OF.get(t.dtype)
+    if code is None:
+        raise TypeError(f"unsupported dtype {t.dtype}")
+    return code
 
 
 def _desc_for(A, B, out_dtype, scale, acc_dtype, variant, flags, tiles) -> ChainDesc:
-    if A.dim() not in (2, 3) or B.dim() not in (2, 3):
+    sa, sb = A.shape, B.shape
+    da, db = len(sa), len(sb)
+    if da not in (2, 3) or db not in (2, 3):
         raise ValueError("A must be [M,K] or [batch,M,K]; B must be [K,N] or [batch,K,N]")
     if not (A.is_contiguous() and B.is_contiguous()):
         raise ValueError("operands must be contiguous (row-major)")
     if A.dtype != B.dtype:
         raise TypeError("A and B must share a dtype")
-    batch = A.shape[0] if A.dim() == 3 else 1
-    M, K = A.shape[-2], A.shape[-1]
-    if B.shape[-2] != K:
-        raise ValueError(f"K mismatch: A has {K}, B has {B.shape[-2]}")
-    N = B.shape[-1]
-    shared_b = B.dim() == 2 and batch > 1
-    if B.dim() == 3 and B.shape[0] != batch:
+    batch = sa[0] if da == 3 else 1
+    M, K = sa[-2], sa[-1]
+    if sb[-2] != K:
+        raise ValueError(f"K mismatch: A has {K}, B has {sb[-2]}")
+    N = sb[-1]
+    shared_b = db == 2 and batch > 1
+    if db == 3 and sb[0] != batch:
         raise ValueError("batch mismatch")
     tm, tn, tk = tiles or (0, 0, 0)
     return make_desc(batch, M, N, K, _dt(A), out_dtype, acc_dtype, scale, shared_b, variant, flags, tm, tn, tk)
@@ -174,7 +178,17 @@ def _desc_for(A, B, out_dtype, scale, acc_dtype, variant, flags, tiles) -> Chain
 
 def _stream_ptr():
     torch = _torch()
-    return C.c_void_p(torch.cuda.current_stream().cuda_stream)
+    return C.c_void_p(torch._C._cuda_getCurrentRawStream(torch.cuda.current_device()))
+
+
+def _on_device(dev, call):
+    """call(stream) on `dev` with dev's current stream: the device is switched only if it is not the current one (a
+    switch there and back costs more than a small launch)."""
+    torch = _torch()
+    if dev.index == torch.cuda.current_device():
+        return call(torch._C._cuda_getCurrentRawStream(dev.index))
+    with torch.cuda.device(dev):
+        return call(torch._C._cuda_getCurrentRawStream(dev.index))
 
 
 def matmul_softmax(A, B, scale: float = 1.0, out=None, out_dtype=None, acc_dtype: int = F32,
@@ -187,20 +201,21 @@ def matmul_softmax(A, B, scale: float = 1.0, out=None, out_dtype=None, acc_dtype
     if out_dtype is None:
         out_dtype = _dt(A)
     d = _desc_for(A, B, out_dtype, scale, acc_dtype, variant, flags, tiles)
+    dev = A.device
     shape = (*A.shape[:-1], B.shape[-1])
     if out is None:
-        out = torch.empty(shape, device=A.device, dtype=torch.float16 if out_dtype == F16 else torch.float32)
-    elif tuple(out.shape) != tuple(shape) or not out.is_contiguous():
+        out = torch.empty(shape, device=dev, dtype=torch.float16 if out_dtype == F16 else torch.float32)
+    elif tuple(out.shape) != shape or not out.is_contiguous():
         raise ValueError("out has the wrong shape or is not contiguous")
     need = workspace_bytes(d)
     if need and (workspace is None or workspace.numel() * workspace.element_size() < need):
-        workspace = torch.empty(need, device=A.device, dtype=torch.uint8)
-    ws_ptr = C.c_void_p(workspace.data_ptr()) if workspace is not None else None
-    ws_len = workspace.numel() * workspace.element_size() if workspace is not None else 0
-    st_ptr = C.c_void_p(status.data_ptr()) if status is not None else None
-    with torch.cuda.device(A.device):
-        _check(lib().wtc_matmul_softmax_launch(C.byref(d), C.c_void_p(A.data_ptr()), C.c_void_p(B.data_ptr()),
-                                               C.c_void_p(out.data_ptr()), ws_ptr, ws_len, _stream_ptr(), st_ptr))
+        workspace = torch.empty(need, device=dev, dtype=torch.uint8)
+    ws_ptr, ws_len = (workspace.data_ptr(), workspace.numel() * workspace.element_size()) if workspace is not None else (None, 0)
+    launch = lib().wtc_matmul_softmax_launch
+    rc = _on_device(dev, lambda stream: launch(d, A.data_ptr(), B.data_ptr(), out.data_ptr(), ws_ptr, ws_len, stream,
+                                               None if status is None else status.data_ptr()))
+    if rc:
+        _check(rc)
     return out
 
 
@@ -305,13 +320,11 @@ def _row_chain(kind, X, out, mean_factor, var_factor):
         out = torch.empty_like(X)
     elif tuple(out.shape) != tuple(X.shape) or out.dtype != X.dtype or not out.is_contiguous():
         raise ValueError("out must match X in shape and dtype and be contiguous")
-    d = RowChainDesc()
-    d.struct_size = C.sizeof(RowChainDesc)
-    d.kind, d.rows, d.N, d.ld_in, d.ld_out = kind, rows, N, 0, 0
-    d.dtype = _dt(X)
-    d.mean_factor, d.var_factor = mean_factor, var_factor
-    with torch.cuda.device(X.device):
-        _check(lib().wtc_row_chain_launch(C.byref(d), C.c_void_p(X.data_ptr()), C.c_void_p(out.data_ptr()), _stream_ptr()))
+    d = RowChainDesc(_ROW_CHAIN_DESC_SIZE, kind, rows, N, 0, 0, _dt(X), mean_factor, var_factor, 0)
+    launch = lib().wtc_row_chain_launch
+    rc = _on_device(X.device, lambda stream: launch(d, X.data_ptr(), out.data_ptr(), stream))
+    if rc:
+        _check(rc)
     return out
 
 
