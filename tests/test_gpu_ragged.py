@@ -149,3 +149,28 @@ def test_rounded_f32_operands_of_ragged_shape(wtc_lib, cuda_dev):
         assert torch.equal(got, same)
         r = oracle.compare(got.cpu().numpy().reshape(-1, N), _ref(A16, B16, 0.1).reshape(-1, N))
         assert r["ok"], r
+
+
+def test_plans_of_few_rows_against_a_wide_matrix(wtc_lib):
+    """128-column tiles up to 64 tiles of 256 columns, 256 beyond; a hint or the forced schedule keeps 256."""
+    w = wtc_lib
+    assert w.plan_query(w.make_desc(1, 16, 4096, 512)).tile_n == 128 and w.plan_query(w.make_desc(1, 16, 16384, 512)).tile_n == 128
+    assert w.plan_query(w.make_desc(1, 16, 16640, 512)).tile_n == 256 and w.plan_query(w.make_desc(1, 256, 8200, 512)).tile_n == 256
+    assert w.plan_query(w.make_desc(1, 16, 4096, 512, tile_n=256)).tile_n == 256
+    assert w.plan_query(w.make_desc(1, 16, 4096, 512, flags=w.FLAG_FORCE_TILED)).tile_n == 256
+    p = w.plan_query(w.make_desc(1, 16, 4104, 512))
+    assert p.kernel == w.KERNEL_TC_TILED and p.workspace_bytes == 16 * 33 * 8
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("M,N,K,out", [(1, 4096, 520, "f16"), (16, 16384, 64, "f16"), (128, 4104, 1000, "f32"), (129, 4096, 72, "f16"), (40, 4097, 333, "f16")])
+def test_few_rows_against_a_wide_matrix(wtc_lib, cuda_dev, M, N, K, out):
+    import torch
+    w = wtc_lib
+    A, B = _operands(1, M, N, K)
+    odt = w.F16 if out == "f16" else w.F32
+    assert w.plan_query(w.make_desc(1, M, N, K, out_dtype=odt)).tile_n == 128
+    got = w.matmul_softmax(torch.from_numpy(A).to(cuda_dev), torch.from_numpy(B).to(cuda_dev), 1 / np.sqrt(K), out_dtype=odt)
+    w.check_device_status()
+    r = oracle.compare(got.cpu().numpy(), oracle.chain(A, B, 1 / np.sqrt(K)))
+    assert r["ok"], r

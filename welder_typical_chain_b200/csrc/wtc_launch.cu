@@ -158,7 +158,10 @@ int resolve(const wtc_chain_desc *in, Resolved &r) {
   // 256-column tile would be padding: 6.4 vs 8.3 us on 8192x128x64) and (b) when 256-column
   // tiles would leave more than half of the SMs without a CTA while the 128-column clusters
   // still all fit the chip at once (measured: 4096x512x1024 12.6 vs 14.5 us, 1024x1024x512
-  // 9.2 vs 11.1 us; but 2048x1024x1024 18.6 vs 14.5 us, where sixteen 8-CTA clusters need two rounds).
+  // 9.2 vs 11.1 us; but 2048x1024x1024 18.6 vs 14.5 us, where sixteen 8-CTA clusters need two rounds), and (c) for rows of
+  // more columns than a cluster holds when there are at most 64 tiles of 256 columns: few rows against a wide matrix are
+  // bound by how many SMs stream it (16x4096x8192 35.6 vs 53.2 us, 128x8192x2048 16.8 vs 22.0, 16x16000x8192 46.8 vs 59.6;
+  // beyond 64 the second column block of a CTA costs more than the idle SMs: 16x18944x512 14.3 vs 13.6).
   r.bn = wtc::kTcBlockN;
   if (d.tile_n == 128) r.bn = 128;
   else if (d.tile_n == 0) {
@@ -168,6 +171,7 @@ int resolve(const wtc_chain_desc *in, Resolved &r) {
     const int64_t nb128 = (d.N + 127) / 128, nb256 = (d.N + 255) / 256;
     if (d.N <= 128) r.bn = 128;
     else if (!(d.flags & WTC_FLAG_FORCE_TILED) && nb128 <= 8 && units * nb256 <= 74 && units <= kResident[nb128]) r.bn = 128;
+    else if (!(d.flags & WTC_FLAG_FORCE_TILED) && nb256 > 8 && units * nb256 <= 64) r.bn = 128;
   }
   r.num_nb = static_cast<int>((d.N + r.bn - 1) / r.bn);
   // tileK is the K depth of one pipeline stage.  64 is the default; 32 and 128 have kernels in the
