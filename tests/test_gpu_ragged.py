@@ -174,3 +174,22 @@ def test_few_rows_against_a_wide_matrix(wtc_lib, cuda_dev, M, N, K, out):
     w.check_device_status()
     r = oracle.compare(got.cpu().numpy(), oracle.chain(A, B, 1 / np.sqrt(K)))
     assert r["ok"], r
+
+
+@pytest.mark.gpu
+def test_workspace_sized_for_wide_tiles_still_serves(wtc_lib, cuda_dev):
+    import torch
+    w = wtc_lib
+    M, N, K = 16, 4104, 512
+    A, B = _operands(1, M, N, K)
+    tA, tB = torch.from_numpy(A).to(cuda_dev), torch.from_numpy(B).to(cuda_dev)
+    d = w.make_desc(1, M, N, K, scale=0.04)
+    old = M * -(-N // 256) * 8
+    assert old < w.workspace_bytes(d)
+    ws = torch.empty(old, device=cuda_dev, dtype=torch.uint8)
+    out = torch.empty((M, N), device=cuda_dev, dtype=torch.float16)
+    assert w.lib().wtc_matmul_softmax_launch(C.byref(d), tA.data_ptr(), tB.data_ptr(), out.data_ptr(), ws.data_ptr(), old, w.current_stream_ptr(), None) == 0
+    w.check_device_status()
+    r = oracle.compare(out.cpu().numpy(), oracle.chain(A, B, 0.04))
+    assert r["ok"], r
+    assert w.lib().wtc_matmul_softmax_launch(C.byref(d), tA.data_ptr(), tB.data_ptr(), out.data_ptr(), ws.data_ptr(), old - 8, w.current_stream_ptr(), None) == -3

@@ -60,6 +60,7 @@ struct Resolved {
   wtc_chain_desc d;  // strides filled in
   wtc_plan_info plan;
   int bn;            // column tile of the tensor-core kernels: 256, or 128 when best.json asks for it
+  bool narrow;       // 128 by the rule for few rows against a wide matrix: a workspace made for 256 still gets 256
   int tm;            // rows of a tile: 128, or best.json's tileM when it is 64 and a kernel exists for it
   int kd;            // K depth of a pipeline stage: 64, or best.json's tileK when it is 32 or 128 and a kernel exists for it
   int num_rb, num_nb, num_kb;
@@ -163,6 +164,7 @@ int resolve(const wtc_chain_desc *in, Resolved &r) {
   // bound by how many SMs stream it (16x4096x8192 35.6 vs 53.2 us, 128x8192x2048 16.8 vs 22.0, 16x16000x8192 46.8 vs 59.6;
   // beyond 64 the second column block of a CTA costs more than the idle SMs: 16x18944x512 14.3 vs 13.6).
   r.bn = wtc::kTcBlockN;
+  r.narrow = false;
   if (d.tile_n == 128) r.bn = 128;
   else if (d.tile_n == 0) {
     // clusters of n CTAs that are resident at once on a 148-SM part (8: measured 15; others: one short of 148 / n)
@@ -171,7 +173,10 @@ int resolve(const wtc_chain_desc *in, Resolved &r) {
     const int64_t nb128 = (d.N + 127) / 128, nb256 = (d.N + 255) / 256;
     if (d.N <= 128) r.bn = 128;
     else if (!(d.flags & WTC_FLAG_FORCE_TILED) && nb128 <= 8 && units * nb256 <= 74 && units <= kResident[nb128]) r.bn = 128;
-    else if (!(d.flags & WTC_FLAG_FORCE_TILED) && nb256 > 8 && units * nb256 <= 64) r.bn = 128;
+    else if (!(d.flags & WTC_FLAG_FORCE_TILED) && nb256 > 8 && units * nb256 <= 64) {
+      r.bn = 128;
+      r.narrow = true;
+    }
   }
   r.num_nb = static_cast<int>((d.N + r.bn - 1) / r.bn);
   // tileK is the K depth of one pipeline stage.  64 is the default; 32 and 128 have kernels in the
@@ -273,6 +278,15 @@ int resolve(const wtc_chain_desc *in, Resolved &r) {
   p.tile_substituted = ((d.tile_m && d.tile_m != p.tile_m) || (d.tile_n && d.tile_n != p.tile_n && d.tile_n < d.N) ||
                         (d.tile_k && d.tile_k != p.tile_k)) ? 1 : 0;
   return WTC_OK;
+}
+
+// The two halves of the sharded form share their statistics' layout with what callers sized for 256-column tiles.
+int widen(Resolved &r) {
+  if (!r.narrow) return WTC_OK;
+  wtc_chain_desc wide = r.d;
+  wide.tile_n = wtc::kTcBlockN;
+  if (!r.b_batched) wide.b_batch_stride = -1;        // (a resolved descriptor holds 0 there)
+  return resolve(&wide, r);
 }
 
 // ---- tensor maps -------------------------------------------------------------
@@ -413,6 +427,15 @@ int launch_resolved(Resolved &r, const void *A, const void *B, void *Out, void *
   const wtc_chain_desc &d = r.d;
   if (d.M == 0 || d.N == 0) return WTC_OK;
   if (!Out || (d.K > 0 && (!A || !B))) return fail(WTC_E_ARG, "null operand pointer");
+  if (mode == 0 && r.narrow && ws_bytes < r.plan.workspace_bytes) {
+    wtc_chain_desc wide = r.d;
+    wide.tile_n = wtc::kTcBlockN;
+    if (!r.b_batched) wide.b_batch_stride = -1;      // (a resolved descriptor holds 0 there)
+    Resolved rw;
+    int rc = resolve(&wide, rw);
+    if (rc) return rc;
+    return launch_resolved(rw, A, B, Out, ws, ws_bytes, row_stats, 0, s, status);
+  }
 
   if (r.trunc) {
     if (mode != 0) return fail(WTC_E_UNSUPPORTED, "the sharded form takes f16 operands");
@@ -616,6 +639,8 @@ int wtc_matmul_softmax_partial_launch(const wtc_chain_desc *desc, const void *A,
   int rc = resolve(desc, r);
   if (rc) return rc;
   if (!r.tc_ok) return fail(WTC_E_UNSUPPORTED, "the sharded form needs f16 operands with 16-byte aligned rows");
+  rc = widen(r);
+  if (rc) return rc;
   return launch_resolved(r, A, B, Out, workspace, workspace_bytes, row_stats, 1, static_cast<cudaStream_t>(stream), device_status);
 }
 
@@ -625,6 +650,8 @@ int wtc_matmul_softmax_finish_launch(const wtc_chain_desc *desc, void *Out, cons
   int rc = resolve(desc, r);
   if (rc) return rc;
   if (!r.tc_ok) return fail(WTC_E_UNSUPPORTED, "the sharded form needs f16 operands/output with 16-byte aligned rows");
+  rc = widen(r);
+  if (rc) return rc;
   if (r.d.M == 0 || r.d.N == 0) return WTC_OK;
   if (!Out || !workspace || !all_stats || num_parts < 1) return fail(WTC_E_ARG, "null pointer or num_parts < 1");
   const int64_t rows = static_cast<int64_t>(r.d.batch) * r.d.M;
