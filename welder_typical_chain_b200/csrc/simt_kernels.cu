@@ -1,5 +1,5 @@
 // SIMT kernels for what the tensor-core path does not take: f32 chains (tcgen05
-// has no f32 MMA), shapes whose row strides are not 16-byte multiples, and the
+// has no f32 MMA), f16 chains too small or too unaligned for it, and the
 // unfused five-kernel pipeline the A/B harness compares the fused kernel with.
 // k is accumulated in ascending order in f32, like a scalar loop nest.
 #include "wtc_kernels.h"
