@@ -534,3 +534,27 @@ def test_operands_ready_keeps_the_order_of_the_stores(w, cuda_dev):
         w.check_device_status()
         torch.cuda.synchronize()
         _check(out.cpu().numpy(), oracle.chain(As[-1].cpu().numpy(), B.cpu().numpy(), 0.05))
+
+
+@pytest.mark.parametrize("N", [512, 509])
+def test_operands_ready_does_not_cover_the_rounded_copies(w, cuda_dev, N):
+    """f32 operands rounded to f16 with WTC_FLAG_OPERANDS_READY: the promise is about the caller's operands; the rounded
+    copies in the workspace are written by the call itself, and the contraction waits for them.  Different operands
+    through one workspace, back to back: every call's result is its own."""
+    import torch
+    M, K, calls = 2000, 512, 6
+    gen = torch.Generator(device=cuda_dev)
+    gen.manual_seed(5)
+    sets = [(torch.randn(M, K, device=cuda_dev, generator=gen), torch.randn(K, N, device=cuda_dev, generator=gen)) for _ in range(calls)]
+    outs = {f: [torch.zeros(M, N, device=cuda_dev, dtype=torch.float16) for _ in range(calls)] for f in (0, w.FLAG_OPERANDS_READY)}
+    ws = torch.empty(w.workspace_bytes(w.make_desc(1, M, N, K, w.F32, w.F16, flags=w.FLAG_MATMUL_F16)), device=cuda_dev, dtype=torch.uint8)
+    for flag, out in outs.items():
+        prepared = [w.PreparedCall(A, B, o, 0.05, workspace=ws, flags=w.FLAG_MATMUL_F16 | flag) for (A, B), o in zip(sets, out)]
+        torch.cuda.synchronize()
+        for _ in range(20):
+            for c in prepared:
+                c.launch(w.current_stream_ptr())
+        w.check_device_status()
+    for (A, B), plain, ready in zip(sets, outs[0], outs[w.FLAG_OPERANDS_READY]):
+        assert torch.equal(plain, ready)
+        _check(ready[:200].cpu().numpy(), oracle.chain(A[:200].half().cpu().numpy(), B.half().cpu().numpy(), 0.05))

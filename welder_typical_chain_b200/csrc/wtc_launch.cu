@@ -128,7 +128,8 @@ int resolve(const wtc_chain_desc *in, Resolved &r) {
     if (d.in_dtype != WTC_F32) return fail(WTC_E_ARG, "WTC_FLAG_MATMUL_F16 needs f32 operands (in_dtype = WTC_F32)");
     wtc_chain_desc inner = d;
     inner.in_dtype = WTC_F16;
-    inner.flags &= ~WTC_FLAG_MATMUL_F16;
+    // (the caller's promise about its operands does not hold for the rounded copies: this call writes them itself)
+    inner.flags &= ~(WTC_FLAG_MATMUL_F16 | WTC_FLAG_OPERANDS_READY);
     inner.lda = round8(d.K); inner.a_batch_stride = d.M * inner.lda;     // rows TMA can read, whatever K and N
     inner.ldb = round8(d.N); inner.b_batch_stride = r.b_batched ? d.K * inner.ldb : -1;
     Resolved ri;
