@@ -112,3 +112,18 @@ def test_static_scratch_rejects_what_does_not_fit(wtc_lib, cuda_dev):
     assert L.wtc_matmul_softmax_launch_static(C.byref(ok), odd, one, one, None, None) == -2
     empty = w.make_desc(1, 0, 64, 64)                        # nothing to compute: accepted like everywhere else
     assert L.wtc_matmul_softmax_launch_static(C.byref(empty), one, one, one, None, None) == 0
+
+
+def test_static_scratch_shares_one_b_among_the_batches(wtc_lib, cuda_dev):
+    """B [K, N] for a batch of A: every batch reads the same B (what lies behind it is other data here)."""
+    import torch
+    w = wtc_lib
+    A, B = oracle.normal((3, 200, 64), 60), oracle.normal((64, 520), 61)
+    behind = torch.full((3 * 64 * 520,), float("nan"), device=cuda_dev, dtype=torch.float16)
+    tB = behind[:64 * 520].view(64, 520)
+    tB.copy_(torch.from_numpy(B).to(cuda_dev))
+    out = torch.empty((3, 200, 520), device=cuda_dev, dtype=torch.float16)
+    w.matmul_softmax_static(torch.from_numpy(A).to(cuda_dev), tB, 0.125, out)
+    w.check_device_status()
+    res = oracle.compare(out.cpu().numpy().reshape(-1, 520), np.concatenate([oracle.chain(a, B, 0.125) for a in A]))
+    assert res["ok"], res

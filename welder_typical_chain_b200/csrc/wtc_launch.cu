@@ -281,12 +281,19 @@ int resolve(const wtc_chain_desc *in, Resolved &r) {
   return WTC_OK;
 }
 
+// A resolved chain's descriptor, to be changed and resolved again: a shared B's stride is 0 there, which would be read as
+// dense batches of B.
+wtc_chain_desc unresolved(const Resolved &r) {
+  wtc_chain_desc d = r.d;
+  if (!r.b_batched) d.b_batch_stride = -1;
+  return d;
+}
+
 // The two halves of the sharded form share their statistics' layout with what callers sized for 256-column tiles.
 int widen(Resolved &r) {
   if (!r.narrow) return WTC_OK;
-  wtc_chain_desc wide = r.d;
+  wtc_chain_desc wide = unresolved(r);
   wide.tile_n = wtc::kTcBlockN;
-  if (!r.b_batched) wide.b_batch_stride = -1;        // (a resolved descriptor holds 0 there)
   return resolve(&wide, r);
 }
 
@@ -429,9 +436,8 @@ int launch_resolved(Resolved &r, const void *A, const void *B, void *Out, void *
   if (d.M == 0 || d.N == 0) return WTC_OK;
   if (!Out || (d.K > 0 && (!A || !B))) return fail(WTC_E_ARG, "null operand pointer");
   if (mode == 0 && r.narrow && ws_bytes < r.plan.workspace_bytes) {
-    wtc_chain_desc wide = r.d;
+    wtc_chain_desc wide = unresolved(r);
     wide.tile_n = wtc::kTcBlockN;
-    if (!r.b_batched) wide.b_batch_stride = -1;      // (a resolved descriptor holds 0 there)
     Resolved rw;
     int rc = resolve(&wide, rw);
     if (rc) return rc;
@@ -829,14 +835,13 @@ int wtc_matmul_softmax_host_submit(const wtc_chain_desc *desc, const void *hostA
     for (int64_t u0 = 0; u0 < units; u0 += per, ++n) {
       const int64_t u1 = u0 + per < units ? u0 + per : units;
       HostSlab &hs = hc.slabs[n];
-      wtc_chain_desc sd = d;
+      wtc_chain_desc sd = unresolved(r);
       hs.b_off = 0; hs.b_len = 0;
       if (by_batch) {
         sd.batch = static_cast<int32_t>(u1 - u0);
         hs.a_off = static_cast<size_t>(u0) * d.a_batch_stride * in_sz;  hs.a_len = static_cast<size_t>(u1 - u0) * d.a_batch_stride * in_sz;
         hs.o_off = static_cast<size_t>(u0) * d.o_batch_stride * out_sz; hs.o_len = static_cast<size_t>(u1 - u0) * d.o_batch_stride * out_sz;
         if (r.b_batched) { hs.b_off = static_cast<size_t>(u0) * d.b_batch_stride * in_sz; hs.b_len = static_cast<size_t>(u1 - u0) * d.b_batch_stride * in_sz; }
-        else sd.b_batch_stride = -1;
       } else {
         const int64_t r0 = u0 * wtc::kTcBlockM, r1 = u1 * wtc::kTcBlockM < d.M ? u1 * wtc::kTcBlockM : d.M;
         sd.M = r1 - r0;
@@ -946,8 +951,9 @@ int wtc_matmul_softmax_launch_static(const wtc_chain_desc *desc, const void *A, 
   if (rc) return rc;
   if (r.d.M == 0 || r.d.N == 0) return WTC_OK;        // nothing to compute, as for the other entry points
   // this entry point always runs the two-pass schedule: size the scratch for the tiles it will use
-  r.d.flags |= WTC_FLAG_FORCE_TILED;
-  rc = resolve(&r.d, r);
+  wtc_chain_desc tiled = unresolved(r);
+  tiled.flags |= WTC_FLAG_FORCE_TILED;
+  rc = resolve(&tiled, r);
   if (rc) return rc;
   if (!r.tc_ok)
     return fail(WTC_E_UNSUPPORTED, "the static-scratch entry point covers the tensor-core two-pass schedule only "
