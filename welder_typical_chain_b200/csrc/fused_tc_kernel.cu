@@ -223,8 +223,12 @@ __device__ __forceinline__ void fold_extreme(const uint32_t (&v)[32], float &m0,
   }
 }
 
+// A row share whose every logit is -inf (masked columns) gets the lowest finite maximum: v - max is then -inf, not NaN, and its
+// probabilities are zeros.  A row that is masked throughout ends as 0 / 0, like any softmax of nothing.
+__device__ __forceinline__ float share_max(float x) { return fmaxf(x, -3.4028235e38f); }
+
 // max (scale >= 0) or min (scale < 0) of a thread's NCH x 32 raw accumulators of which the
-// first `valid` exist, times c2: the row share's largest logit in the log2 domain
+// first `valid` exist, times c2: the row share's largest logit in the log2 domain (-inf: no column exists)
 template <int NCH>
 __device__ __forceinline__ float share_extreme(const uint32_t (&r)[NCH][32], int valid, float c2) {
   const bool pos = c2 >= 0.f;
@@ -234,11 +238,11 @@ __device__ __forceinline__ float share_extreme(const uint32_t (&r)[NCH][32], int
     if (pos) {
 #pragma unroll
       for (int c = 0; c < NCH; ++c) fold_extreme<true>(r[c], m0, m1, m2, m3);
-      return fmaxf(fmaxf(m0, m1), fmaxf(m2, m3)) * c2;
+      return share_max(fmaxf(fmaxf(m0, m1), fmaxf(m2, m3)) * c2);
     }
 #pragma unroll
     for (int c = 0; c < NCH; ++c) fold_extreme<false>(r[c], m0, m1, m2, m3);
-    return fminf(fminf(m0, m1), fminf(m2, m3)) * c2;
+    return share_max(fminf(fminf(m0, m1), fminf(m2, m3)) * c2);
   }
   if (valid <= 0) return -INFINITY;
   // the row's last tile: whole chunks like everywhere else, element by element only in the one that the row ends in (the CTAs of a
@@ -255,7 +259,7 @@ __device__ __forceinline__ float share_extreme(const uint32_t (&r)[NCH][32], int
         if (c * 32 + i < valid) m0 = pos ? fmaxf(m0, __uint_as_float(r[c][i])) : fminf(m0, __uint_as_float(r[c][i]));
     }
   }
-  return (pos ? fmaxf(fmaxf(m0, m1), fmaxf(m2, m3)) : fminf(fminf(m0, m1), fminf(m2, m3))) * c2;
+  return share_max((pos ? fmaxf(fmaxf(m0, m1), fmaxf(m2, m3)) : fminf(fminf(m0, m1), fminf(m2, m3))) * c2);
 }
 
 // e = 2^(v * c2 - m) in place for a chunk of 32 accumulators of which the first `valid` exist (the others become 0); adds to the sums
@@ -533,7 +537,7 @@ fused_tc_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__
 #pragma unroll
           for (int c = NCH / 2; c < NCH; ++c) fold_extreme<false>(r[c], m0, m1, m2, m3);
         }
-        m_half = (pos ? fmaxf(fmaxf(m0, m1), fmaxf(m2, m3)) : fminf(fminf(m0, m1), fminf(m2, m3))) * c2;
+        m_half = share_max((pos ? fmaxf(fmaxf(m0, m1), fmaxf(m2, m3)) : fminf(fminf(m0, m1), fminf(m2, m3))) * c2);
       } else {
 #pragma unroll
         for (int c = 0; c < NCH; ++c) {
