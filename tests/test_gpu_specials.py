@@ -59,3 +59,27 @@ def test_masked_columns_are_zeros(wtc_lib, cuda_dev, M, N, K, out, flag, scale):
     w.check_device_status()
     bad = torch.isnan(got).any(-1)
     assert bool(bad[7]) and int(bad.sum()) == 1
+
+
+@pytest.mark.parametrize("M,N,K,out,flag,scale", _FORMS)
+def test_logits_far_from_zero(wtc_lib, cuda_dev, M, N, K, out, flag, scale):
+    """Logits of 1e8 to 1e12: one-hot rows, and equal logits give equal probabilities."""
+    import torch
+    w = wtc_lib
+    flags = getattr(w, flag) if flag else 0
+    odt = w.F16 if out == "f16" else w.F32
+    sign = 1.0 if scale > 0 else -1.0
+    for mag in (3000.0, 20000.0):
+        A, B = ((x * mag).clamp(-60000, 60000).half() for x in _operands(torch, cuda_dev, M, N, K, 2))
+        L = sign * (A.double() @ B.double())
+        top = L.topk(2, -1).values
+        clear = top[:, 0] - top[:, 1] > 2.0 ** -16 * top[:, 0]         # rows whose largest logit is no tie within f32 sums
+        assert clear.float().mean() > 0.9
+        got = w.matmul_softmax(A, B, sign, out_dtype=odt, flags=flags)
+        w.check_device_status()
+        want = torch.nn.functional.one_hot(L.argmax(-1), N)
+        assert bool((got.double() - want)[clear].abs().le(2.0 ** -22).all())
+        A, B = torch.full_like(A, mag), torch.full_like(B, mag)
+        got = w.matmul_softmax(A, B, sign, out_dtype=odt, flags=flags)
+        w.check_device_status()
+        assert bool((got.double() * N - 1).abs().le(2.0 ** -10 if out == "f16" else 2.0 ** -20).all())

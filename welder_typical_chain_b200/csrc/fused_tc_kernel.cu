@@ -223,28 +223,36 @@ __device__ __forceinline__ void fold_extreme(const uint32_t (&v)[32], float &m0,
   }
 }
 
-// A row share whose every logit is -inf (masked columns) gets the lowest finite maximum: v - max is then -inf, not NaN, and its
-// probabilities are zeros.  A row that is masked throughout ends as 0 / 0, like any softmax of nothing.
-__device__ __forceinline__ float share_max(float x) { return fmaxf(x, -3.4028235e38f); }
+constexpr float kLowest = -3.4028235e38f;
+// The share's largest logit (log2 domain) from its raw extreme.  A share whose every logit is -inf (masked columns) gets the lowest
+// finite maximum: v - max is then -inf, not NaN, and its probabilities are zeros.  A row that is masked throughout ends as 0 / 0,
+// like any softmax of nothing.
+__device__ __forceinline__ float share_max(float extreme, float c2) { return fmaxf(extreme * c2, kLowest); }
+
+// A share's exponents are 2^(v * c2 - m), one FMA a value.  The rounding of the maximum m is the same factor on all of the share's
+// values and cancels in the quotient; but when the logits lie so far from zero that it amounts to more than 2^8 (an f16 ends at
+// 2^16, an f32 at 2^128), c2 gives way to the power of two below it, whose product with the extreme is exact: neighbouring f32
+// sums are at least a factor of 2^16 apart there, whatever the factor.  Such shares take the forms' general path.  (The extreme
+// is taken a second time there: kept in a register it costs every tile, 14.00 against 13.97 us for 4096 x 1024 x 1024.)
+__device__ __forceinline__ bool far_from_zero(float m) { return fabsf(m) >= 268435456.f && m > kLowest; }
+__device__ __forceinline__ float far_factor(float c2) { return __uint_as_float(__float_as_uint(c2) & 0xFF800000u); }
 
 // max (scale >= 0) or min (scale < 0) of a thread's NCH x 32 raw accumulators of which the
-// first `valid` exist, times c2: the row share's largest logit in the log2 domain (-inf: no column exists)
+// first `valid` > 0 exist: times c2, the row share's largest logit in the log2 domain
 template <int NCH>
-__device__ __forceinline__ float share_extreme(const uint32_t (&r)[NCH][32], int valid, float c2) {
-  const bool pos = c2 >= 0.f;
+__device__ __forceinline__ float share_extreme(const uint32_t (&r)[NCH][32], int valid, bool pos) {
   if (valid == NCH * 32) {
     float m0 = __uint_as_float(r[0][0]), m1 = __uint_as_float(r[0][1]);
     float m2 = __uint_as_float(r[0][2]), m3 = __uint_as_float(r[0][3]);
     if (pos) {
 #pragma unroll
       for (int c = 0; c < NCH; ++c) fold_extreme<true>(r[c], m0, m1, m2, m3);
-      return share_max(fmaxf(fmaxf(m0, m1), fmaxf(m2, m3)) * c2);
+      return fmaxf(fmaxf(m0, m1), fmaxf(m2, m3));
     }
 #pragma unroll
     for (int c = 0; c < NCH; ++c) fold_extreme<false>(r[c], m0, m1, m2, m3);
-    return share_max(fminf(fminf(m0, m1), fminf(m2, m3)) * c2);
+    return fminf(fminf(m0, m1), fminf(m2, m3));
   }
-  if (valid <= 0) return -INFINITY;
   // the row's last tile: whole chunks like everywhere else, element by element only in the one that the row ends in (the CTAs of a
   // cluster wait for this one: 24 x 1021 x 1021 x 64 45.9 and 41.5 us, with f32 output 54.4 and 47.2)
   float m0 = __uint_as_float(r[0][0]), m1 = m0, m2 = m0, m3 = m0;
@@ -259,7 +267,7 @@ __device__ __forceinline__ float share_extreme(const uint32_t (&r)[NCH][32], int
         if (c * 32 + i < valid) m0 = pos ? fmaxf(m0, __uint_as_float(r[c][i])) : fminf(m0, __uint_as_float(r[c][i]));
     }
   }
-  return share_max((pos ? fmaxf(fmaxf(m0, m1), fmaxf(m2, m3)) : fminf(fminf(m0, m1), fminf(m2, m3))) * c2);
+  return pos ? fmaxf(fmaxf(m0, m1), fmaxf(m2, m3)) : fminf(fminf(m0, m1), fminf(m2, m3));
 }
 
 // e = 2^(v * c2 - m) in place for a chunk of 32 accumulators of which the first `valid` exist (the others become 0); adds to the sums
@@ -511,7 +519,7 @@ fused_tc_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__
       const int col0 = nb * BN + half * HC;
       const int valid = max(0, min(HC, p.N - col0));
       uint32_t r[NCH][32];
-      float m_half;
+      float extreme = 0.f;
       if (valid == HC && !p.round_logits_f16) {
         // whole share, no rounding: the second half of the loads is in flight while the
         // extreme of the first half is taken
@@ -537,7 +545,7 @@ fused_tc_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__
 #pragma unroll
           for (int c = NCH / 2; c < NCH; ++c) fold_extreme<false>(r[c], m0, m1, m2, m3);
         }
-        m_half = share_max((pos ? fmaxf(fmaxf(m0, m1), fmaxf(m2, m3)) : fminf(fminf(m0, m1), fminf(m2, m3))) * c2);
+        extreme = pos ? fmaxf(fmaxf(m0, m1), fmaxf(m2, m3)) : fminf(fminf(m0, m1), fminf(m2, m3));
       } else {
 #pragma unroll
         for (int c = 0; c < NCH; ++c) {
@@ -554,11 +562,13 @@ fused_tc_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__
 #pragma unroll
             for (int i = 0; i < 32; ++i) r[c][i] = __float_as_uint(__half2float(__float2half_rn(__uint_as_float(r[c][i]))));
         }
-        m_half = share_extreme<NCH>(r, valid, c2);
+        if (valid > 0) extreme = share_extreme<NCH>(r, valid, c2 >= 0.f);
       }
+      const float m_half = valid > 0 ? share_max(extreme, c2) : -INFINITY;
       // ---- e = 2^(v - m_half) in place, row sum; each chunk goes back over its logits ----
       float s0 = 0.f, s1 = 0.f, s2 = 0.f, s3 = 0.f;
-      if (valid == HC) {
+      const bool far = far_from_zero(m_half);
+      if (valid == HC && !__any_sync(0xffffffffu, far)) {        // (a warp stores to tensor memory together)
 #pragma unroll
         for (int c = 0; c < NCH; ++c) {
 #pragma unroll
@@ -574,12 +584,13 @@ fused_tc_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__
           tmem_st_32x32b_x32(tbase + c * 32, r[c]);
         }
       } else {
+        const float factor = far ? far_factor(c2) : c2, offset = far ? share_extreme<NCH>(r, valid, c2 >= 0.f) * factor : m_half;
 #pragma unroll
         for (int c = 0; c < NCH; ++c) {
 #pragma unroll
           for (int i = 0; i < 32; ++i) {
             float e = 0.f;
-            if (c * 32 + i < valid) e = ex2_approx(fmaf(__uint_as_float(r[c][i]), c2, -m_half));
+            if (c * 32 + i < valid) e = ex2_approx(fmaf(__uint_as_float(r[c][i]), factor, -offset));
             s0 += e;
             r[c][i] = __float_as_uint(e);
           }
@@ -726,11 +737,12 @@ fused_tc_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__
 #pragma unroll
             for (int i = 0; i < 32; ++i) r[c][i] = __float_as_uint(__half2float(__float2half_rn(__uint_as_float(r[c][i]))));
         }
-        const float m_part = share_extreme<NCH>(r, valid, c2);
+        const float m_part = valid > 0 ? share_max(share_extreme<NCH>(r, valid, c2 >= 0.f), c2) : -INFINITY;
         if (lead) WTC_STAMP(p, TS_MAX);
         // ---- e = 2^(v - m_part) in place, row sum ----
         float s0 = 0.f, s1 = 0.f, s2 = 0.f, s3 = 0.f;
-        if (valid == HC) {
+        const bool far = far_from_zero(m_part);
+        if (valid == HC && !far) {
 #pragma unroll
           for (int c = 0; c < NCH; ++c)
 #pragma unroll
@@ -744,8 +756,9 @@ fused_tc_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__
               r[c][i + 2] = __float_as_uint(e2); r[c][i + 3] = __float_as_uint(e3);
             }
         } else {
+          const float factor = far ? far_factor(c2) : c2, offset = far ? share_extreme<NCH>(r, valid, c2 >= 0.f) * factor : m_part;
 #pragma unroll
-          for (int c = 0; c < NCH; ++c) exp_chunk(r[c], valid - c * 32, c2, m_part, s0, s1, s2, s3);   // (columns that do not exist: 0)
+          for (int c = 0; c < NCH; ++c) exp_chunk(r[c], valid - c * 32, factor, offset, s0, s1, s2, s3);   // (columns that do not exist: 0)
         }
         const float sum = (s0 + s1) + (s2 + s3);
         if (lead) WTC_STAMP(p, TS_EXP);
@@ -975,12 +988,13 @@ fused_tc_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__
         }
         continue;
       }
-      const float m_half = share_extreme<NCH>(r, valid, c2);
+      const float m_half = valid > 0 ? share_max(share_extreme<NCH>(r, valid, c2 >= 0.f), c2) : -INFINITY;
       if (lead && it == 0) WTC_STAMP(p, TS_MAX);
 
       // ---- e = 2^(v - m_half) in place, row sum ----
       float s0 = 0.f, s1 = 0.f, s2 = 0.f, s3 = 0.f;
-      if (valid == HC) {
+      const bool far = far_from_zero(m_half);
+      if (valid == HC && !far) {
 #pragma unroll
         for (int c = 0; c < NCH; ++c)
 #pragma unroll
@@ -994,9 +1008,10 @@ fused_tc_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__
             r[c][i + 2] = __float_as_uint(e2); r[c][i + 3] = __float_as_uint(e3);
           }
       } else {
+        const float factor = far ? far_factor(c2) : c2, offset = far ? share_extreme<NCH>(r, valid, c2 >= 0.f) * factor : m_half;
 #pragma unroll
         for (int c = 0; c < NCH; ++c)
-          if (c * 32 < valid) exp_chunk(r[c], valid - c * 32, c2, m_half, s0, s1, s2, s3);   // (what lies behind is not stored)
+          if (c * 32 < valid) exp_chunk(r[c], valid - c * 32, factor, offset, s0, s1, s2, s3);   // (what lies behind is not stored)
       }
       const float sum = (s0 + s1) + (s2 + s3);
       if (lead && it == 0) WTC_STAMP(p, TS_EXP);
