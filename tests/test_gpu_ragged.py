@@ -84,6 +84,29 @@ def test_ragged_matches_the_checker(wtc_lib, cuda_dev, batch, M, N, K, out, kw):
 
 
 @pytest.mark.gpu
+@pytest.mark.parametrize("batch,M,N,K,rounded", [(1, 300, 3001, 64, False), (2, 257, 2049, 100, False), (1, 16, 4097, 333, False), (1, 700, 2056, 61, False),
+                                                 (1, 150, 20001, 72, False), (1, 300, 3001, 251, True), (1, 130, 2304, 67, True)])
+def test_long_ragged_rows_round_a_probability_once(wtc_lib, cuda_dev, batch, M, N, K, rounded):
+    """f16 probabilities of rows of more than eight column tiles: within half an f16 step of the value in 64 bits, as from the
+    SIMT kernel (an f16 value relative to a tile's maximum on the way would cost another half)."""
+    import torch
+    w = wtc_lib
+    gen = torch.Generator(device=cuda_dev)
+    gen.manual_seed(N)
+    A = torch.randn((batch, M, K) if batch > 1 else (M, K), device=cuda_dev, generator=gen)
+    B = torch.randn((batch, K, N) if batch > 1 else (K, N), device=cuda_dev, generator=gen)
+    A16, B16 = A.half(), B.half()
+    flags = w.FLAG_MATMUL_F16 if rounded else 0
+    assert w.plan_query(w.make_desc(batch, M, N, K, w.F32 if rounded else w.F16, w.F16, flags=flags)).kernel == w.KERNEL_TC_TILED
+    for scale in (1.0 / K ** 0.5, -0.3):
+        P = ((A16.double() @ B16.double()) * scale).softmax(-1)
+        got = w.matmul_softmax(A if rounded else A16, B if rounded else B16, scale, out_dtype=w.F16, flags=flags)
+        w.check_device_status()
+        # half a step of f16 (2^-11 relative, 2^-25 among the subnormals) and the f32 sums of K products below 30
+        assert bool((got.double() - P).abs().le((2.0 ** -11 + 2.0 ** -24 * (30 * K ** 0.5 + 16)) * P + 2.0 ** -25).all())
+
+
+@pytest.mark.gpu
 def test_ragged_strided_output_and_neighbours(wtc_lib, cuda_dev):
     """A padded output: the columns between rows, and what lies before and behind, stay untouched; odd row starts."""
     import torch

@@ -41,7 +41,8 @@
 // PAIR: two CTAs issue one 256-row tcgen05 cta_group::2 MMA (tiled flavour, long K).
 // OUT32: f32 probabilities.
 // DIRECT: output rows that TMA cannot store (a stride that is no multiple of 16 bytes): the warp
-// that staged a tile writes its rows itself (split form).
+// that staged a tile writes its rows itself (split form).  Tiled with f16 output it runs twice, statistics
+// first (TcParams::stats_pass), so that a probability is rounded once.
 // KD, TM: K depth of a pipeline stage (64; 32 or 128 on request) and rows of a tile (128;
 // 64 on request, tcgen05.mma with M = 64) -- the schedule's tileK and tileM.
 //
@@ -294,6 +295,12 @@ __device__ __forceinline__ void exp_chunk(uint32_t (&v)[32], int valid, float c2
   }
 }
 
+// (max, sum) pairs of disjoint column sets of a row -> the pair of their union (-inf: the empty set)
+__device__ __forceinline__ float2 combine_pairs(float2 a, float2 b) {
+  const float m = fmaxf(a.x, b.x);
+  return make_float2(m, (a.x == -INFINITY ? 0.f : a.y * ex2_approx(a.x - m)) + (b.x == -INFINITY ? 0.f : b.y * ex2_approx(b.x - m)));
+}
+
 // 32 values times f, rounded to f16 pairs
 __device__ __forceinline__ void scale_pack(const uint32_t (&r)[32], float f, uint32_t (&h)[16]) {
 #pragma unroll
@@ -310,6 +317,7 @@ fused_tc_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__
   constexpr bool RELAY = L::RELAY;
   constexpr bool SINGLE = L::SINGLE;
   constexpr int OUT_TILES = L::kOutTiles;
+  constexpr bool TWO_PASS = DIRECT && !CLUSTER && !OUT32;   // p.stats_pass
   constexpr int HC = L::kHalfCols;      // columns per epilogue thread
   constexpr int NCH = HC / 32;          // 32-column chunks per epilogue thread
   constexpr int kEpiThreads = (RELAY || SINGLE) ? 512 : 256;
@@ -935,6 +943,16 @@ fused_tc_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__
       const int ab = it & 1;
       const int par = it & 1;
       const uint32_t tile_phase = (it >> 1) & 1;
+      float2 row_part = make_float2(-INFINITY, 0.f);     // second pass: every other tile's statistics of my row, the other half takes the rest
+      if (TWO_PASS && p.stats_pass == 2) {
+        if (it == 0) grid_dependency_wait();             // (the first pass wrote them)
+        const int row = rb * TM + row_in_tile;
+        if (row < p.M) {
+          const float2 *st = p.tile_stats + (static_cast<int64_t>(b) * p.M + row) * p.num_nb;
+          for (int t = half; t < p.num_nb; t += 2) row_part = combine_pairs(row_part, st[t]);
+        }
+        __syncwarp();
+      }
       if (CLUSTER && lead) mbar_expect_tx(&stats_bar[par], cluster_n * BM * 8);
       if (!mbar_wait(&accum_full[ab], tile_phase)) { record_failure(p.status, WTC_DEV_TIMEOUT_ACCUM); break; }
       tc_fence_after_sync();
@@ -1017,13 +1035,23 @@ fused_tc_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__
       if (lead && it == 0) WTC_STAMP(p, TS_EXP);
 
       // ---- the two halves of a row meet through shared memory ----
-      *mine = make_float2(m_half, sum);
+      *mine = TWO_PASS && p.stats_pass == 2 ? row_part : make_float2(m_half, sum);
       named_bar_sync(1 + q, 64);
       const float2 o = *other;
       named_bar_sync(1 + q, 64);                 // both have read: the slots may be reused
       const float lm = fmaxf(m_half, o.x);       // tile-row max (log2 domain)
       float f;                                     // what my e values still have to be multiplied by
-      if (CLUSTER) {
+      if (TWO_PASS && p.stats_pass == 1) {
+        const int row = rb * TM + row_in_tile;
+        if (half == 0 && row < p.M)
+          p.tile_stats[(static_cast<int64_t>(b) * p.M + row) * p.num_nb + nb] = combine_pairs(make_float2(m_half, sum), o);
+        __syncwarp();
+        continue;
+      }
+      if (TWO_PASS && p.stats_pass == 2) {
+        const float2 all = combine_pairs(row_part, o);
+        f = ex2_approx(m_half - all.x) * rcp_approx(all.y);
+      } else if (CLUSTER) {
         const float ll = (m_half == -INFINITY ? 0.f : sum * ex2_approx(m_half - lm)) +
                          (o.x == -INFINITY ? 0.f : o.y * ex2_approx(o.x - lm));
         // ... and the CTAs of the cluster through each other's shared memory
@@ -1129,7 +1157,7 @@ fused_tc_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__
           }
         }
       }
-      if (!CLUSTER) {
+      if (!CLUSTER && !(TWO_PASS && p.stats_pass == 2)) {
         // tile statistics: max of the tile row, sum of the stored values of both halves
         mine->y = sum_r;
         named_bar_sync(1 + q, 64);

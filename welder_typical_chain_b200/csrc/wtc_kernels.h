@@ -36,6 +36,9 @@ struct TcParams {
   int *status;     // device status word (0 = ok)
   // rows of the output that TMA cannot store (strides that are no multiple of 16 bytes): written from the staging tiles
   int direct_out;
+  // ... of the tiled flavour with f16 output, in two passes: 1 leaves only the tiles' statistics, 2 contracts again and
+  // writes probabilities, rounded once, from all statistics of a row
+  int stats_pass;
   void *out;
   int64_t ldo, o_batch_stride;
 #ifdef WTC_BRINGUP

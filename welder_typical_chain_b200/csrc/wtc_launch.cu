@@ -71,6 +71,10 @@ struct Resolved {
   bool ragged;
   size_t copy_a, copy_b;
   bool direct_out;
+  // ... of the tiled flavour with f16 output: these chains round a probability once, as the SIMT kernel does, so no values relative
+  // to a tile's maximum are stored on the way; the tiles' statistics come from a first pass over the contraction, the
+  // probabilities from a second (error against 64 bits 2.1e-4 of the result; with f16 values rescaled 2.7e-4)
+  bool two_pass;
   // WTC_FLAG_MATMUL_F16: f32 operands are first rounded to dense f16 copies at the head of the
   // workspace, then `inner` (the same chain on f16 operands) runs on the copies
   bool trunc = false;
@@ -208,7 +212,7 @@ int resolve(const wtc_chain_desc *in, Resolved &r) {
   // pointers off their 16-byte boundaries, runs there.
   const bool tiled_row = r.num_nb > 8 || (d.flags & WTC_FLAG_FORCE_TILED);
   r.copy_a = r.copy_b = 0;
-  r.direct_out = false;
+  r.direct_out = r.two_pass = false;
   r.ragged = !tc_shape && d.in_dtype == WTC_F16 && d.M > 0 && d.N > 0 && d.K > 0 && d.variant == WTC_VARIANT_FUSED &&
              !(d.flags & WTC_FLAG_FORCE_SIMT) && static_cast<double>(d.batch) * d.M * d.N * d.K >= kRaggedMinWork &&
              wtc::simt_fused_takes(simt_params(r)) && static_cast<int64_t>(d.batch) * r.num_rb * r.num_nb < 0x7fffffff &&
@@ -219,7 +223,8 @@ int resolve(const wtc_chain_desc *in, Resolved &r) {
     r.num_kb = static_cast<int>((d.K + r.kd - 1) / r.kd);
     if (!mult8(d.K) || !mult8(d.lda) || !mult8(d.a_batch_stride)) r.copy_a = align256(static_cast<size_t>(d.batch) * d.M * round8(d.K) * 2);
     if (!mult8(d.ldb) || !mult8(d.b_batch_stride)) r.copy_b = align256(static_cast<size_t>(r.b_batched ? d.batch : 1) * d.K * round64(d.N) * 2);
-    r.direct_out = !mult8(d.N) || !mult8(d.ldo) || !mult8(d.o_batch_stride);      // (a TMA store fills the last 16 bytes of a row)
+    r.two_pass = tiled_row && d.out_dtype == WTC_F16;
+    r.direct_out = !mult8(d.N) || !mult8(d.ldo) || !mult8(d.o_batch_stride) || r.two_pass;      // (a TMA store fills the last 16 bytes of a row)
   }
 
   if (d.variant == WTC_VARIANT_BASELINE) {
@@ -580,8 +585,14 @@ int launch_resolved(Resolved &r, const void *A, const void *B, void *Out, void *
     if (!ws || ws_bytes < need) return fail(WTC_E_WORKSPACE, "tiled schedule needs %zu workspace bytes, got %zu", need, ws_bytes);
     p.num_items = d.batch * r.num_rb * r.num_nb;
     p.tile_stats = static_cast<float2 *>(ws);
+    p.stats_pass = r.two_pass ? 1 : 0;
     e = wtc::launch_tiled_partial(tmA, tmB, tmO, p, r.bn, sms, s, &info);
     if (e != cudaSuccess) return cuda_fail(e, "tiled kernel launch");
+    if (r.two_pass) {
+      p.stats_pass = 2;
+      e = wtc::launch_tiled_partial(tmA, tmB, tmO, p, r.bn, sms, s, &info);
+      return e == cudaSuccess ? WTC_OK : cuda_fail(e, "tiled kernel launch, second pass");
+    }
     const int64_t rows = static_cast<int64_t>(d.batch) * d.M;
     if (mode == 1) {
       if (!row_stats) return fail(WTC_E_ARG, "partial launch needs a row_stats buffer");
