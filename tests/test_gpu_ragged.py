@@ -216,3 +216,30 @@ def test_workspace_sized_for_wide_tiles_still_serves(wtc_lib, cuda_dev):
     r = oracle.compare(out.cpu().numpy(), oracle.chain(A, B, 0.04))
     assert r["ok"], r
     assert w.lib().wtc_matmul_softmax_launch(C.byref(d), tA.data_ptr(), tB.data_ptr(), out.data_ptr(), ws.data_ptr(), old - 8, w.current_stream_ptr(), None) == -3
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("M,N,K,kw", [
+    (1000, 333, 64, {}), (1000, 333, 256, {}), (1000, 333, 257, {}), (1000, 333, 320, {}), (700, 1021, 512, {}), (700, 1021, 1023, {}), (300, 3001, 1000, {}),
+    (2000, 129, 777, {}), (8200, 1001, 600, {}), (500, 1000, 1001, {}), (400, 3000, 515, {}), (300, 1021, 4001, {}), (700, 1001, 1001, {"rounded": True}),
+])
+def test_f32_results_of_ragged_chains_are_no_further_off(wtc_lib, cuda_dev, M, N, K, kw):
+    """f16 operands, f32 probabilities: the error against 64 bits is at most the SIMT kernel's (the same call with that kernel
+    forced), whatever K; sums of more than 256 products are put together from partial ones."""
+    import torch
+    w = wtc_lib
+    flags = w.FLAG_MATMUL_F16 if kw.get("rounded") else 0
+    off = {"tc": 0.0, "simt": 0.0}
+    for seed in range(3):
+        gen = torch.Generator(device=cuda_dev)
+        gen.manual_seed(seed)
+        A, B = torch.randn(M, K, device=cuda_dev, generator=gen), torch.randn(K, N, device=cuda_dev, generator=gen)
+        a, b = (A, B) if flags else (A.half(), B.half())
+        scale = 1.0 / K ** 0.5
+        P = ((A.half().double() @ B.half().double()) * scale).softmax(-1)
+        assert w.plan_query(w.make_desc(1, M, N, K, w.F32 if flags else w.F16, w.F32, flags=flags)).kernel != w.KERNEL_SIMT_FUSED
+        for name, extra in (("tc", 0), ("simt", w.FLAG_FORCE_SIMT)):
+            got = w.matmul_softmax(a, b, scale, out_dtype=w.F32, flags=flags | extra)
+            w.check_device_status()
+            off[name] += float((got.double() - P).norm() / P.norm())
+    assert off["tc"] <= off["simt"], off

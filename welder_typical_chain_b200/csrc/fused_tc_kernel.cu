@@ -318,6 +318,9 @@ fused_tc_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__
   constexpr bool SINGLE = L::SINGLE;
   constexpr int OUT_TILES = L::kOutTiles;
   constexpr bool TWO_PASS = DIRECT && !CLUSTER && !OUT32;   // p.stats_pass
+  // Partial sums (p.sum_kb): the tensor core's running f32 sum loses a little with every step, and beyond some 256 products more
+  // than FMAs do (K = 1023: 1.7e-6 of the result against 1.05e-6).  Added in registers, sums of 256 keep the error below theirs.
+  constexpr bool PARTIAL = DIRECT && OUT32;
   constexpr int HC = L::kHalfCols;      // columns per epilogue thread
   constexpr int NCH = HC / 32;          // 32-column chunks per epilogue thread
   constexpr int kEpiThreads = (RELAY || SINGLE) ? 512 : 256;
@@ -885,40 +888,45 @@ fused_tc_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__
       int it = 0;
       bool ok = true;
       for (int w = first; w < p.num_items && ok; w += stride, ++it) {
-        const int ab = it & 1;
-        if (!mbar_wait(&accum_empty[ab], ((it >> 1) & 1) ^ 1)) { record_failure(p.status, WTC_DEV_TIMEOUT_TMEM); ok = false; break; }
-        tc_fence_after_sync();
-        if (it == 8) WTC_STAMP(p, TS_LOADED);
-        const uint32_t d_tmem = tmem_base + ab * BN;
-        for (int kb = 0; kb < p.num_kb; ++kb) {
-          if (!landed && !mbar_wait(&full[s], ph)) { record_failure(p.status, WTC_DEV_TIMEOUT_FULL); ok = false; break; }
+        int kb = 0;
+        do {                            // once, or a round for each partial sum (`it` counts accumulators then)
+          const int ab = it & 1;
+          if (!mbar_wait(&accum_empty[ab], ((it >> 1) & 1) ^ 1)) { record_failure(p.status, WTC_DEV_TIMEOUT_TMEM); ok = false; break; }
           tc_fence_after_sync();
-          if (it == 0 && kb == 0) WTC_STAMP(p, TS_FULL0);
-          uint64_t da = a_desc0 + ((s * L::kStageBytes) >> 4);
-          uint64_t db = b_desc0 + ((s * L::kStageBytes) >> 4);
+          if (it == 8) WTC_STAMP(p, TS_LOADED);
+          const uint32_t d_tmem = tmem_base + ab * BN;
+          const int kb0 = PARTIAL ? kb : 0, kb1 = PARTIAL && p.sum_kb ? min(kb + p.sum_kb, p.num_kb) : p.num_kb;
+          for (; kb < kb1; ++kb) {
+            if (!landed && !mbar_wait(&full[s], ph)) { record_failure(p.status, WTC_DEV_TIMEOUT_FULL); ok = false; break; }
+            tc_fence_after_sync();
+            if (it == 0 && kb == 0) WTC_STAMP(p, TS_FULL0);
+            uint64_t da = a_desc0 + ((s * L::kStageBytes) >> 4);
+            uint64_t db = b_desc0 + ((s * L::kStageBytes) >> 4);
 #pragma unroll
-          for (int k = 0; k < BK / 16; ++k) {
-            if (PAIR) umma_f16_ss_pair(d_tmem, da, db, idesc, (kb | k) != 0);
-            else umma_f16_ss(d_tmem, da, db, idesc, (kb | k) != 0);
-            da += (k == 3 ? TM * 128 - 3 * kAKstep : kAKstep) >> 4;   // after four steps: the second 64-column block of a 128-deep stage
-            db += kBKstep >> 4;
+            for (int k = 0; k < BK / 16; ++k) {
+              if (PAIR) umma_f16_ss_pair(d_tmem, da, db, idesc, (kb | k) != 0);
+              else umma_f16_ss(d_tmem, da, db, idesc, ((kb - kb0) | k) != 0);
+              da += (k == 3 ? TM * 128 - 3 * kAKstep : kAKstep) >> 4;   // after four steps: the second 64-column block of a 128-deep stage
+              db += kBKstep >> 4;
+            }
+            // while those MMAs drain: has the next stage landed already?  (The ring runs on
+            // across tiles, so "next" is the same barrier whichever tile it belongs to.)
+            const uint32_t s1 = s + 1 == STAGES ? 0 : s + 1;
+            const uint32_t ph1 = s1 == 0 ? ph ^ 1 : ph;
+            landed = mbar_try_wait(&full[s1], ph1);
+            // frees the stage (in both CTAs of a pair) once these MMAs have read it
+            if (PAIR) umma_commit_pair(&empty[s], pair_mask);
+            else umma_commit(&empty[s]);
+            s = s1; ph = ph1;
           }
-          // while those MMAs drain: has the next stage landed already?  (The ring runs on
-          // across tiles, so "next" is the same barrier whichever tile it belongs to.)
-          const uint32_t s1 = s + 1 == STAGES ? 0 : s + 1;
-          const uint32_t ph1 = s1 == 0 ? ph ^ 1 : ph;
-          landed = mbar_try_wait(&full[s1], ph1);
-          // frees the stage (in both CTAs of a pair) once these MMAs have read it
-          if (PAIR) umma_commit_pair(&empty[s], pair_mask);
-          else umma_commit(&empty[s]);
-          s = s1; ph = ph1;
-        }
-        if (ok) {
-          if (PAIR) umma_commit_pair(&accum_full[ab], pair_mask);
-          else umma_commit(&accum_full[ab]);
-          if (it == 0) WTC_STAMP(p, TS_MMA_DONE);
-          if (it == 8) WTC_STAMP(p, TS_MAX);
-        }
+          if (ok) {
+            if (PAIR) umma_commit_pair(&accum_full[ab], pair_mask);
+            else umma_commit(&accum_full[ab]);
+            if (it == 0) WTC_STAMP(p, TS_MMA_DONE);
+            if (it == 8) WTC_STAMP(p, TS_MAX);
+          }
+          if (PARTIAL && kb < p.num_kb) ++it;
+        } while (PARTIAL && ok && kb < p.num_kb);
       }
     }
     __syncwarp();
@@ -937,12 +945,14 @@ fused_tc_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__
     const float2 *other = &pair[(half ^ 1) * BM + row_in_tile];
     const float c2 = p.c2;
     int it = 0;
+    const int sums = PARTIAL && p.sum_kb ? (p.num_kb + p.sum_kb - 1) / p.sum_kb : 1;     // accumulators of a tile
     uint32_t gcount = 0;                         // staging groups committed so far by this warp
     for (int w = first; w < p.num_items; w += stride, ++it) {
       int b, rb, nb; decode(w, b, rb, nb);
-      const int ab = it & 1;
+      const int acc = PARTIAL ? it * sums : it;          // the tile's first accumulator
+      const int ab = acc & 1;
       const int par = it & 1;
-      const uint32_t tile_phase = (it >> 1) & 1;
+      const uint32_t tile_phase = (it >> 1) & 1;         // of the statistics' barriers
       float2 row_part = make_float2(-INFINITY, 0.f);     // second pass: every other tile's statistics of my row, the other half takes the rest
       if (TWO_PASS && p.stats_pass == 2) {
         if (it == 0) grid_dependency_wait();             // (the first pass wrote them)
@@ -954,7 +964,7 @@ fused_tc_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__
         __syncwarp();
       }
       if (CLUSTER && lead) mbar_expect_tx(&stats_bar[par], cluster_n * BM * 8);
-      if (!mbar_wait(&accum_full[ab], tile_phase)) { record_failure(p.status, WTC_DEV_TIMEOUT_ACCUM); break; }
+      if (!mbar_wait(&accum_full[ab], (acc >> 1) & 1)) { record_failure(p.status, WTC_DEV_TIMEOUT_ACCUM); break; }
       tc_fence_after_sync();
       if (p.operands_ready && it == 0) grid_dependency_wait();   // nothing of this warp has touched global memory yet
       if (lead && it == 0) WTC_STAMP(p, TS_ACCUM);
@@ -978,6 +988,31 @@ fused_tc_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__
       tmem_ld_wait();
       tc_fence_before_sync();
       release_accumulator(ab);
+      if (PARTIAL && sums > 1) {
+        bool landed = true;
+        for (int i = 1; i < sums; ++i) {
+          const int at = (acc + i) & 1;
+          if (!(landed = mbar_wait(&accum_full[at], ((acc + i) >> 1) & 1))) break;
+          tc_fence_after_sync();
+          const uint32_t from = tmem_base + (static_cast<uint32_t>(q * 32) << 16) + at * BN + half * HC;
+#pragma unroll
+          for (int c = 0; c < 2 * NCH; ++c) {
+            if (c * 16 < valid) {
+              uint32_t part[16];
+              tmem_ld_32x32b_x16(from + c * 16, part);
+              tmem_ld_wait();
+#pragma unroll
+              for (int e = 0; e < 16; ++e) {
+                uint32_t &v = r[c >> 1][(c & 1) * 16 + e];
+                v = __float_as_uint(__uint_as_float(v) + __uint_as_float(part[e]));
+              }
+            }
+          }
+          tc_fence_before_sync();
+          release_accumulator(at);
+        }
+        if (!landed) { record_failure(p.status, WTC_DEV_TIMEOUT_ACCUM); break; }
+      }
       if (lead && it == 0) WTC_STAMP(p, TS_LOADED);
       if (p.round_logits_f16) {
 #pragma unroll

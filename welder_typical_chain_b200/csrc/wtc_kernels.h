@@ -39,6 +39,8 @@ struct TcParams {
   // ... of the tiled flavour with f16 output, in two passes: 1 leaves only the tiles' statistics, 2 contracts again and
   // writes probabilities, rounded once, from all statistics of a row
   int stats_pass;
+  // ... with f32 output: K blocks summed in one tensor-memory accumulator; the epilogue adds these partial sums (0: all of them)
+  int sum_kb;
   void *out;
   int64_t ldo, o_batch_stride;
 #ifdef WTC_BRINGUP

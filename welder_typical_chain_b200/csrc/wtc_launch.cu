@@ -75,6 +75,8 @@ struct Resolved {
   // to a tile's maximum are stored on the way; the tiles' statistics come from a first pass over the contraction, the
   // probabilities from a second (error against 64 bits 2.1e-4 of the result; with f16 values rescaled 2.7e-4)
   bool two_pass;
+  // ... with f32 output and long K: the K blocks of a partial sum, else 0
+  int sum_kb;
   // WTC_FLAG_MATMUL_F16: f32 operands are first rounded to dense f16 copies at the head of the
   // workspace, then `inner` (the same chain on f16 operands) runs on the copies
   bool trunc = false;
@@ -90,6 +92,9 @@ int64_t round64(int64_t v) { return (v + 63) & ~static_cast<int64_t>(63); }
 // Multiply-adds from which a ragged f16 chain goes to the tensor cores: below, the SIMT row kernel's one launch is faster
 // than an operand copy and a chain (500 x 333 x 64: 9.2 against 10.0 us; 1000 x 1001 x 16: 12.3 against 10.5 us).
 constexpr double kRaggedMinWork = 12 << 20;
+// K blocks of 64 that a ragged chain with f32 output sums in one accumulator.  Error against 64 bits of the result, N(0, 1) operands
+// and scale 1 / sqrt(K), over the SIMT kernel's: 0.64 at K = 128, 0.90 at 256; in one sum 1.06 at 320, 1.16 at 512, 1.6 at 1023.
+constexpr int kRaggedSumKb = 4;
 
 wtc::SimtParams simt_params(const Resolved &r) {
   wtc::SimtParams s;
@@ -213,6 +218,7 @@ int resolve(const wtc_chain_desc *in, Resolved &r) {
   const bool tiled_row = r.num_nb > 8 || (d.flags & WTC_FLAG_FORCE_TILED);
   r.copy_a = r.copy_b = 0;
   r.direct_out = r.two_pass = false;
+  r.sum_kb = 0;
   r.ragged = !tc_shape && d.in_dtype == WTC_F16 && d.M > 0 && d.N > 0 && d.K > 0 && d.variant == WTC_VARIANT_FUSED &&
              !(d.flags & WTC_FLAG_FORCE_SIMT) && static_cast<double>(d.batch) * d.M * d.N * d.K >= kRaggedMinWork &&
              wtc::simt_fused_takes(simt_params(r)) && static_cast<int64_t>(d.batch) * r.num_rb * r.num_nb < 0x7fffffff &&
@@ -224,7 +230,8 @@ int resolve(const wtc_chain_desc *in, Resolved &r) {
     if (!mult8(d.K) || !mult8(d.lda) || !mult8(d.a_batch_stride)) r.copy_a = align256(static_cast<size_t>(d.batch) * d.M * round8(d.K) * 2);
     if (!mult8(d.ldb) || !mult8(d.b_batch_stride)) r.copy_b = align256(static_cast<size_t>(r.b_batched ? d.batch : 1) * d.K * round64(d.N) * 2);
     r.two_pass = tiled_row && d.out_dtype == WTC_F16;
-    r.direct_out = !mult8(d.N) || !mult8(d.ldo) || !mult8(d.o_batch_stride) || r.two_pass;      // (a TMA store fills the last 16 bytes of a row)
+    r.sum_kb = d.out_dtype == WTC_F32 && r.num_kb > kRaggedSumKb ? kRaggedSumKb : 0;
+    r.direct_out = !mult8(d.N) || !mult8(d.ldo) || !mult8(d.o_batch_stride) || r.two_pass || r.sum_kb;      // (a TMA store fills the last 16 bytes of a row)
   }
 
   if (d.variant == WTC_VARIANT_BASELINE) {
@@ -566,6 +573,7 @@ int launch_resolved(Resolved &r, const void *A, const void *B, void *Out, void *
     p.operands_ready = (d.flags & WTC_FLAG_OPERANDS_READY) && !r.copy_a && !r.copy_b ? 1 : 0;   // (the copies are earlier work on the stream)
     p.out_f32 = out32;
     p.direct_out = r.direct_out;
+    p.sum_kb = r.sum_kb;
     p.out = Out;
     p.ldo = d.ldo; p.o_batch_stride = d.o_batch_stride;
     p.stage_k = r.kd;
