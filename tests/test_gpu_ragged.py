@@ -185,6 +185,14 @@ def test_plans_of_few_rows_against_a_wide_matrix(wtc_lib):
     assert p.kernel == w.KERNEL_TC_TILED and p.workspace_bytes == 16 * 33 * 8
 
 
+def test_pairs_on_request_keep_their_tiles(wtc_lib):
+    """WTC_FLAG_PAIR pairs CTAs whenever there are two row blocks: 256-column tiles, whatever the number of tiles."""
+    w = wtc_lib
+    p = w.plan_query(w.make_desc(1, 256, 4096, 1024, flags=w.FLAG_PAIR))
+    assert (p.tile_n, p.stages) == (256, 6) and p.workspace_bytes == 256 * 16 * 8
+    assert w.plan_query(w.make_desc(1, 256, 4096, 1024)).tile_n == 128
+
+
 @pytest.mark.gpu
 @pytest.mark.parametrize("M,N,K,out", [(1, 4096, 520, "f16"), (16, 16384, 64, "f16"), (128, 4104, 1000, "f32"), (129, 4096, 72, "f16"), (40, 4097, 333, "f16")])
 def test_few_rows_against_a_wide_matrix(wtc_lib, cuda_dev, M, N, K, out):

@@ -183,7 +183,7 @@ int resolve(const wtc_chain_desc *in, Resolved &r) {
     const int64_t nb128 = (d.N + 127) / 128, nb256 = (d.N + 255) / 256;
     if (d.N <= 128) r.bn = 128;
     else if (!(d.flags & WTC_FLAG_FORCE_TILED) && nb128 <= 8 && units * nb256 <= 74 && units <= kResident[nb128]) r.bn = 128;
-    else if (!(d.flags & WTC_FLAG_FORCE_TILED) && nb256 > 8 && units * nb256 <= 64) {
+    else if (!(d.flags & (WTC_FLAG_FORCE_TILED | WTC_FLAG_PAIR)) && nb256 > 8 && units * nb256 <= 64) {      // (CTA pairs have 256-column tiles)
       r.bn = 128;
       r.narrow = true;
     }
