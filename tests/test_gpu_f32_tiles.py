@@ -14,6 +14,28 @@ def test_launch_counts(wtc_lib):
     assert w.plan_query(w.make_desc(1, 128, 128, 128, w.F32, w.F32)).launches == 1
 
 
+def test_plans_describe_the_tile_kernel(wtc_lib):
+    """Tile, threads, stages, shared memory, cluster and launches of the kernel that runs, not of the row kernel."""
+    w = wtc_lib
+
+    def fields(*shape, **kw):
+        p = w.plan_query(w.make_desc(*shape, w.F32, w.F32, **kw))
+        return p.tile_m, p.tile_n, p.tile_k, p.cluster_n, p.threads, p.stages, p.launches
+
+    assert fields(1, 4096, 1024, 1024) == (128, 256, 16, 4, 256, 4, 1)
+    p = w.plan_query(w.make_desc(1, 4096, 1024, 1024, w.F32, w.F32))
+    assert p.smem_bytes == 4 * (4 * 16 * (132 + 256) + (4 + 16 + 2) * 128)       # four stages of A (padded rows) and B, the row statistics
+    assert fields(1, 300, 4096, 1024)[3] == 1 and fields(1, 300, 4096, 1024)[6] == 2
+    assert fields(1, 128, 128, 128) == (16, 128, 64, 1, 256, 0, 1)
+    # batches whose rows do not follow one another: a row softmax each
+    d = w.make_desc(3, 300, 4096, 256, w.F32, w.F32)
+    assert w.plan_query(d).launches == 2
+    d.o_batch_stride = 301 * 4096
+    assert w.plan_query(d).launches == 4
+    # f16 output: rows of more than eight tiles stay with the row kernel
+    assert w.plan_query(w.make_desc(1, 300, 4096, 1024, w.F32, w.F16)).stages == 0
+
+
 @pytest.mark.gpu
 @pytest.mark.parametrize("batch,M,N,K,shared", [
     (1, 4096, 1024, 96, False),      # 128 x 256 tiles, clusters of four

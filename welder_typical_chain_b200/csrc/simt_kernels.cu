@@ -533,6 +533,13 @@ cudaError_t launch_tile(const float *A, const float *B, void *Out, const SimtPar
   return vecb ? launch_tile_v<TM, WR, WC, true>(A, B, Out, p, logits_only, s) : launch_tile_v<TM, WR, WC, false>(A, B, Out, p, logits_only, s);
 }
 
+template <int TM, int WR, int WC> SimtPlan tile_plan() {
+  using T = TileShape<TM, WR, WC>;
+  return SimtPlan{T::BM, T::BN, kTileK, 1, T::kThreads, static_cast<int>(T::kSmem), T::kStages, 1};
+}
+
+bool stacked_densely(const SimtParams &p) { return p.batch == 1 || p.o_batch_stride == static_cast<int64_t>(p.M) * p.ldo; }
+
 cudaError_t launch_tiles(const void *A, const void *B, void *Out, const SimtParams &p, cudaStream_t s) {
   const float *a = static_cast<const float *>(A), *b = static_cast<const float *>(B);
   const int c = pick_tile(p);
@@ -543,7 +550,7 @@ cudaError_t launch_tiles(const void *A, const void *B, void *Out, const SimtPara
   else if (c == 2) e = launch_tile<8, 2, 2>(a, b, Out, p, logits_only, s);
   else e = launch_tile<4, 2, 2>(a, b, Out, p, logits_only, s);
   if (e != cudaSuccess || !logits_only) return e;
-  const bool dense = p.batch == 1 || p.o_batch_stride == static_cast<int64_t>(p.M) * p.ldo;
+  const bool dense = stacked_densely(p);
   const int64_t rows = dense ? static_cast<int64_t>(p.batch) * p.M : p.M;
   for (int i = 0; i < (dense ? 1 : p.batch) && e == cudaSuccess; ++i) {
     float *o = static_cast<float *>(Out) + i * p.o_batch_stride;
@@ -556,8 +563,14 @@ cudaError_t launch_tiles(const void *A, const void *B, void *Out, const SimtPara
 
 bool simt_fused_takes(const SimtParams &p) { return pick_rows(p, kRowLimit) != 0; }
 
-int simt_fused_launches(const SimtParams &p) {
-  return use_tiles(p, pick_rows(p, kRowLimit)) && p.N > 8 * kTileChoices[pick_tile(p)].bn ? 2 : 1;
+SimtPlan simt_fused_plan(const SimtParams &p) {
+  if (!use_tiles(p, pick_rows(p, kRowLimit))) return SimtPlan{16, p.N, kKChunk, 1, kSimtThreads, 0, 0, 1};
+  const int c = pick_tile(p);
+  const int nb = (p.N + kTileChoices[c].bn - 1) / kTileChoices[c].bn;
+  SimtPlan r = c == 0 ? tile_plan<16, 2, 4>() : c == 1 ? tile_plan<8, 2, 4>() : c == 2 ? tile_plan<8, 2, 2>() : tile_plan<4, 2, 2>();
+  r.cluster_n = nb > 8 ? 1 : nb;
+  r.launches = nb > 8 ? 1 + (stacked_densely(p) ? 1 : p.batch) : 1;
+  return r;
 }
 
 cudaError_t launch_simt_fused(const void *A, const void *B, void *Out, const SimtParams &p, cudaStream_t s) {

@@ -122,7 +122,10 @@ struct SimtParams {
 };
 cudaError_t launch_simt_fused(const void *A, const void *B, void *Out, const SimtParams &p, cudaStream_t s);
 bool simt_fused_takes(const SimtParams &p);     // whether a row is short enough for the SIMT path
-int simt_fused_launches(const SimtParams &p);
+// What a call runs: the row kernel (stages 0), or the register-tiled f32 kernel and, for rows of more than eight column tiles,
+// a row softmax over its logits (one launch per batch where the output's batches are not densely stacked).
+struct SimtPlan { int tile_m, tile_n, tile_k, cluster_n, threads, smem_bytes, stages, launches; };
+SimtPlan simt_fused_plan(const SimtParams &p);
 // Unfused five-kernel pipeline: matmul -> row max -> exp -> row sum -> divide,
 // with C32[M,N], max[M], E[M,N], sum[M] in global memory (workspace).
 cudaError_t launch_simt_unfused(const void *A, const void *B, void *Out, void *workspace, const SimtParams &p,

@@ -284,9 +284,16 @@ int resolve(const wtc_chain_desc *in, Resolved &r) {
     }
   } else {
     p.kernel = WTC_KERNEL_SIMT_FUSED;
-    p.launches = (d.M > 0 && d.N > 0) ? wtc::simt_fused_launches(simt_params(r)) : 0;
-    p.threads = 256;
-    p.tile_m = 16; p.tile_n = static_cast<int32_t>(d.N); p.tile_k = 64;
+    if (d.M > 0 && d.N > 0) {
+      const wtc::SimtPlan v = wtc::simt_fused_plan(simt_params(r));
+      p.launches = v.launches;
+      p.cluster_n = v.cluster_n;
+      p.threads = v.threads; p.stages = v.stages; p.smem_bytes = v.smem_bytes;
+      p.tile_m = v.tile_m; p.tile_n = v.tile_n; p.tile_k = v.tile_k;
+    } else {
+      p.threads = 256;
+      p.tile_m = 16; p.tile_n = static_cast<int32_t>(d.N); p.tile_k = 64;
+    }
   }
   p.tile_substituted = ((d.tile_m && d.tile_m != p.tile_m) || (d.tile_n && d.tile_n != p.tile_n && d.tile_n < d.N) ||
                         (d.tile_k && d.tile_k != p.tile_k)) ? 1 : 0;

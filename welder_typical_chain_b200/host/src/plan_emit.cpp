@@ -112,6 +112,10 @@ std::string launchText(const ir::ChainSpec &s, const PlanResult &pr) {
     o << "gpu.launch @" << name << " blocks(" << grid << ") cluster(" << cluster << ") threads(" << threads << ", 1, 1) workgroup(" << smem
       << ")  // " << note << "\n";
   };
+  // rows TMA cannot take: f16 output of the tiled schedule then comes from two passes over the contraction
+  const bool twoPass = p.kernel == WTC_KERNEL_TC_TILED && (s.K % 8 || s.N % 8) && s.outType == "f16";
+  if ((p.kernel == WTC_KERNEL_TC_CLUSTER && p.launches > 1) || (p.kernel == WTC_KERNEL_TC_TILED && p.launches > 2))
+    launch("copy_operands_kernel", "elementwise, 8 columns a thread", "1, 1, 1", 256, "0", "operands as f16 rows that TMA can read, in the workspace");
   switch (p.kernel) {
     case WTC_KERNEL_TC_CLUSTER:
       launch("fused_tc_kernel_cluster", "min(" + std::to_string(s.batch * rb) + " row blocks, resident clusters) x " + std::to_string(p.cluster_n),
@@ -122,12 +126,26 @@ std::string launchText(const ir::ChainSpec &s, const PlanResult &pr) {
     case WTC_KERNEL_TC_TILED:
       launch("fused_tc_kernel_tiled", "min(" + std::to_string(s.batch * rb * nb) + " tiles, SMs)", "1, 1, 1", p.threads,
              std::to_string(p.stages) + " stages x 48 KiB operands + 32 KiB f16 staging",
-             "persistent; writes exp(v - tile max) and per-tile (max,sum), workspace " + std::to_string(p.workspace_bytes) + " B");
-      launch("rescale_rows_kernel", std::to_string(s.batch * s.M) + " rows", "1, 1, 1", 256, std::to_string(nb * 4) + " B",
+             std::string(twoPass ? "persistent; per-tile (max,sum) only" : "persistent; writes exp(v - tile max) and per-tile (max,sum)") + ", workspace " +
+                 std::to_string(p.workspace_bytes) + " B");
+      if (twoPass)
+        launch("fused_tc_kernel_tiled", "min(" + std::to_string(s.batch * rb * nb) + " tiles, SMs)", "1, 1, 1", p.threads,
+               std::to_string(p.stages) + " stages x 48 KiB operands + 32 KiB f16 staging", "the contraction again, probabilities from all (max,sum) of a row");
+      else
+        launch("rescale_rows_kernel", std::to_string(s.batch * s.M) + " rows", "1, 1, 1", 256, std::to_string(nb * 4) + " B",
              "log-sum-exp over the tiles of a row, rescale in place");
       break;
     case WTC_KERNEL_SIMT_FUSED:
-      launch("simt_fused_kernel", "ceil(rows / R)", "1, 1, 1", 256, "R x (64 + N) f32", "exact f32 accumulate, k ascending; one warp per row in the softmax");
+      if (p.stages > 0) {
+        const std::string tile = std::to_string(p.tile_m) + " x " + std::to_string(p.tile_n);
+        launch("simt_tile_kernel", std::to_string(s.batch) + " x ceil(rows / " + std::to_string(p.tile_m) + ") x ceil(columns / " + std::to_string(p.tile_n) + ")",
+               std::to_string(p.cluster_n) + ", 1, 1", p.threads, std::to_string(p.smem_bytes) + " B",
+               "exact f32 accumulate, k ascending; " + tile + " register tiles, " + std::to_string(p.stages) + " stages of 16 k" +
+                   (p.launches > 1 ? "; logits to the output" : "; row max and sum swapped through DSMEM"));
+        if (p.launches > 1) launch("row_softmax", std::to_string(s.batch * s.M) + " rows", "1, 1, 1", 256, "0", "softmax of the logits in place");
+      } else {
+        launch("simt_fused_kernel", "ceil(rows / R)", "1, 1, 1", 256, "R x (64 + N) f32", "exact f32 accumulate, k ascending; one warp per row in the softmax");
+      }
       break;
     default:
       launch("unfused_matmul_kernel", "ceil(rows / 8)", "1, 1, 1", 256, "8 x 64 f32", "C32 = scale * A.B -> global");
