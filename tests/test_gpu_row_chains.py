@@ -145,3 +145,27 @@ def test_row_softmax_in_place_and_at_the_limits(wtc_lib, cuda_dev):
         for r in (0, 1, 3, 4, 8):
             assert torch.allclose(out[r].double(), ref[r], rtol=4e-6, atol=0), (N, r)
         assert torch.isnan(out[2]).all()
+
+
+@pytest.mark.gpu
+def test_more_short_rows_than_a_cluster_grid_could_hold(wtc_lib, cuda_dev):
+    """2^28 and a few rows of eight elements: more than an eighth of the largest grid, and still several rows a warp (a CTA a
+    row would take a hundred times as long as the traffic)."""
+    import torch
+    w = wtc_lib
+    rows, N = (1 << 28) + 5, 8
+    X = torch.zeros(rows, N, device=cuda_dev, dtype=torch.float16)
+    for piece in X.split(1 << 24):
+        piece.normal_()
+    out = torch.empty_like(X)
+    w.row_softmax(X, out=out)
+    torch.cuda.synchronize()
+    for at in (0, rows // 2, rows - 1000):
+        P = X[at:at + 1000].double().softmax(-1)
+        assert bool((out[at:at + 1000].double() - P).abs().le(2.0 ** -11 * P + 2.0 ** -24).all())
+    start, end = torch.cuda.Event(enable_timing=True), torch.cuda.Event(enable_timing=True)
+    start.record()
+    w.row_softmax(X, out=out)
+    end.record()
+    torch.cuda.synchronize()
+    assert start.elapsed_time(end) < 10 * 2 * X.numel() * 2 / 6e9       # ten times what 6 TB/s take

@@ -403,7 +403,7 @@ cudaError_t launch_rows(const void *X, void *Out, int64_t rows, int N, int64_t l
     return cudaGetLastError();
   }
   constexpr int kNv = 8, one = 512 * kNv * V;           // vectors a thread and elements a CTA of a cluster
-  const int cluster = N <= 2 * one ? 2 : (N <= 4 * one ? 4 : 8);
+  const int cluster = N <= 4 * one ? 4 : 8;              // (rows of up to two CTAs' worth went above)
   cudaLaunchConfig_t cfg = {};
   cfg.gridDim = dim3(g * cluster, 1, 1);
   cfg.blockDim = dim3(threads_for((N + cluster - 1) / cluster, kNv), 1, 1);
@@ -427,7 +427,8 @@ cudaError_t launch_typed(const void *X, void *Out, int64_t rows, int N, int64_t 
   const bool vec = N % V == 0 && (ld_in * ES) % 16 == 0 && (ld_out * ES) % 16 == 0 && (x & 15) == 0 && (o & 15) == 0;
   // every row's input and output lie equally far from a 16-byte boundary: whole vectors on both sides
   const bool together = x % ES == 0 && (x & 15) == (o & 15) && ((ld_in - ld_out) * ES) % 16 == 0;
-  const bool fits = N <= 8 * 512 * 8 * V && rows <= 0x7fffffff / 8;      // a cluster of eight CTAs holds the row
+  // a CTA holds the row, or a cluster of eight (whose grid is eight times the rows)
+  const bool fits = N <= 512 * 16 * V || (N <= 8 * 512 * 8 * V && rows <= 0x7fffffff / 8);
   if (fits && vec) return launch_rows<KIND, F16, false>(X, Out, rows, N, ld_in, ld_out, c1, c2, s);
   if (fits && together) return launch_rows<KIND, F16, true>(X, Out, rows, N, ld_in, ld_out, c1, c2, s);
   row_chain_block_kernel<KIND, F16, F16><<<static_cast<unsigned>(rows), 256, 0, s>>>(X, Out, N, ld_in, ld_out, c1, c2);
