@@ -169,3 +169,16 @@ def test_more_short_rows_than_a_cluster_grid_could_hold(wtc_lib, cuda_dev):
     end.record()
     torch.cuda.synchronize()
     assert start.elapsed_time(end) < 10 * 2 * X.numel() * 2 / 6e9       # ten times what 6 TB/s take
+
+
+@pytest.mark.parametrize("N", [64, 61, 1024, 4096, 5000, 5003, 16384, 32000, 40000])
+def test_f32_row_softmax_far_from_zero(wtc_lib, cuda_dev, N):
+    """Equal values of any size give equal probabilities, values of 1e9 and more one-hot rows, whatever the alignment."""
+    import torch
+    w = wtc_lib
+    for value in (torch.finfo(torch.float32).min, torch.finfo(torch.float32).max, 3e38, 1e10, -1e10, 1e7):
+        out = w.row_softmax(torch.full((5, N), value, device=cuda_dev))
+        assert bool((out.double() * N - 1).abs().le(2.0 ** -20).all()), value
+    X = torch.randn((9, N), device=cuda_dev) * 3e9          # neighbouring f32 values lie 64 and more apart here
+    want = torch.softmax(X.double(), -1)
+    assert bool((w.row_softmax(X).double() - want).abs().le(2.0 ** -22).all())

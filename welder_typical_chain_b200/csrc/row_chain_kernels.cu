@@ -100,8 +100,8 @@ template <bool F16> __device__ __forceinline__ uint4 load_raw(const void *base, 
 // for the sum, once for the result: the special-function unit has the headroom, the memory system
 // does not.
 //
-// The exponent is fma(x, log2 e, -max * log2 e); (x - max) * log2 e in the ragged f32 form, which
-// stays exact at the maximum for rows near the type's limits.  KIND 2 is the
+// The exponent is fma(x, log2 e, -max * log2 e) of f16 rows, (x - max) * log2 e of f32 ones: there the
+// product's rounding alone passes an f32's exponent range from |max| = 2^31 on.  KIND 2 is the
 // softmax of the f32 chain's logits (X and Out the same buffer): expf and a division, as the fused
 // f32 kernel computes them.
 template <int KIND, bool F16, int NV, bool RAGGED, bool PACKED, typename Reduce>
@@ -155,7 +155,7 @@ __device__ __forceinline__ void chain_on_row(const void *X, void *Out, int64_t i
     }
     m = reduce(m, true);
     const float mb = m * kLog2e;
-    auto ex = [&](float x) { return KIND == 2 ? expf(x - m) : RAGGED && !F16 ? ex2_approx((x - m) * kLog2e) : ex2_approx(fmaf(x, kLog2e, -mb)); };   // exp(x - max); -inf padding gives 0
+    auto ex = [&](float x) { return KIND == 2 ? expf(x - m) : !F16 ? ex2_approx((x - m) * kLog2e) : ex2_approx(fmaf(x, kLog2e, -mb)); };   // exp(x - max); -inf padding gives 0
     float s = 0.f;
     if (RAGGED) {
       xh = ex(xh); xt = ex(xt);
