@@ -44,6 +44,36 @@ def test_ragged_plans(wtc_lib):
     assert w.plan_query(w.make_desc(1, 500, 60001, 64)).kernel == w.KERNEL_SIMT_FUSED      # refused at launch, as before
 
 
+def test_padded_rows_of_a_are_read_in_place(wtc_lib):
+    """Any K, with rows of A on 16-byte strides: nothing to copy; f32 operands are rounded into such rows, once."""
+    w = wtc_lib
+    p = w.plan_query(w.make_desc(1, 1000, 1000, 61, lda=64))
+    assert (p.kernel, p.launches, p.workspace_bytes) == (w.KERNEL_TC_CLUSTER, 1, 0)
+    p = w.plan_query(w.make_desc(1, 1000, 1000, 61, in_dtype=w.F32, flags=w.FLAG_MATMUL_F16))
+    same = w.plan_query(w.make_desc(1, 1000, 1000, 64, in_dtype=w.F32, flags=w.FLAG_MATMUL_F16))
+    assert p.kernel == w.KERNEL_TC_CLUSTER and p.launches == same.launches == 2
+    assert p.workspace_bytes == 1000 * 64 * 2 + -(-61 * 1000 * 2 // 256) * 256
+
+
+@pytest.mark.gpu
+def test_padded_rows_of_a_hide_what_lies_between_them(wtc_lib, cuda_dev):
+    """K = 61 in rows of 64: the three elements behind each row are NaN and no part of the sums."""
+    import torch
+    w = wtc_lib
+    M, N, K = 700, 1000, 61
+    A, B = _operands(1, M, N, K)
+    tA = torch.full((M, 64), float("nan"), device=cuda_dev, dtype=torch.float16)
+    tA[:, :K] = torch.from_numpy(A).to(cuda_dev)
+    tB = torch.from_numpy(B).to(cuda_dev)
+    out = torch.empty((M, N), device=cuda_dev, dtype=torch.float16)
+    d = w.make_desc(1, M, N, K, scale=0.1, lda=64)
+    assert w.plan_query(d).launches == 1
+    assert w.lib().wtc_matmul_softmax_launch(C.byref(d), tA.data_ptr(), tB.data_ptr(), out.data_ptr(), None, 0, w.current_stream_ptr(), None) == 0
+    w.check_device_status()
+    r = oracle.compare(out.cpu().numpy(), oracle.chain(A, B, 0.1))
+    assert r["ok"], r
+
+
 @pytest.mark.gpu
 @pytest.mark.parametrize("batch,M,N,K,out,kw", [
     (1, 2000, 129, 64, "f16", {}),          # 128-column tiles, one column in the second

@@ -227,7 +227,8 @@ int resolve(const wtc_chain_desc *in, Resolved &r) {
     r.kd = wtc::kTcBlockK; r.tm = wtc::kTcBlockM;           // these kernels exist for the default tiles only
     r.num_rb = static_cast<int>((d.M + wtc::kTcBlockM - 1) / wtc::kTcBlockM);
     r.num_kb = static_cast<int>((d.K + r.kd - 1) / r.kd);
-    if (!mult8(d.K) || !mult8(d.lda) || !mult8(d.a_batch_stride)) r.copy_a = align256(static_cast<size_t>(d.batch) * d.M * round8(d.K) * 2);
+    // (strides count: a K that is no multiple of 8 is only an extent of A's map, which fills zeros behind it)
+    if (!mult8(d.lda) || !mult8(d.a_batch_stride)) r.copy_a = align256(static_cast<size_t>(d.batch) * d.M * round8(d.K) * 2);
     if (!mult8(d.ldb) || !mult8(d.b_batch_stride)) r.copy_b = align256(static_cast<size_t>(r.b_batched ? d.batch : 1) * d.K * round64(d.N) * 2);
     r.two_pass = tiled_row && d.out_dtype == WTC_F16;
     r.sum_kb = d.out_dtype == WTC_F32 && r.num_kb > kRaggedSumKb ? kRaggedSumKb : 0;
