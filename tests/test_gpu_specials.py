@@ -83,3 +83,20 @@ def test_logits_far_from_zero(wtc_lib, cuda_dev, M, N, K, out, flag, scale):
         got = w.matmul_softmax(A, B, sign, out_dtype=odt, flags=flags)
         w.check_device_status()
         assert bool((got.double() * N - 1).abs().le(2.0 ** -10 if out == "f16" else 2.0 ** -20).all())
+
+
+@pytest.mark.parametrize("out", ["f16", "f32"])
+@pytest.mark.parametrize("M,N", [(888, 2304), (889, 2304), (3, 5000), (111, 20000), (112, 20000)])
+def test_row_rescale_on_both_sides_of_its_rule(wtc_lib, cuda_dev, M, N, out):
+    """One vector a thread beyond 888 CTAs, four up to there; a CTA per row, and several."""
+    import torch
+    w = wtc_lib
+    A, B = (x.half() for x in _operands(torch, cuda_dev, M, N, 64, 3))
+    odt = w.F16 if out == "f16" else w.F32
+    assert w.plan_query(w.make_desc(1, M, N, 64, out_dtype=odt)).kernel == w.KERNEL_TC_TILED
+    got = w.matmul_softmax(A, B, 0.125, out_dtype=odt)
+    w.check_device_status()
+    P = _chain64(A, B, 0.125)
+    # f16: the value relative to its tile's maximum and the rescaled one are both rounded
+    tol = 2.0 ** -10 if out == "f16" else 2.0 ** -24 * 100
+    assert bool((got.double() - P).abs().le(tol * P + 2.0 ** -23).all())

@@ -40,11 +40,18 @@ __global__ void row_stats_kernel(const float2 *__restrict__ tile_stats, float2 *
 // columns (a multiple of 256) after working out the row's total for itself.
 //
 // Pure traffic: the output read and written once more.  Rows go from the last to the first, because
-// the tiled kernel in front wrote the last ones last: up to an L2 of them need no read from memory.
-// Four vectors a thread are in flight, and what is written is not kept from the rows still to come.
-// Whole chain, before and with all three: 8192 x 8192 x 256 111.5 and 100.3 us, 4096 x 32000 x 256 212.8
-// and 195.6, f32 8192 x 8192 x 256 179.2 and 162.7; order and loads without the streaming stores 101.5, 207.7, 167.8.
-constexpr int kRescaleVecs = 4;
+// the tiled kernel in front wrote the last ones last: up to an L2 of them need no read from memory;
+// and what is written is not kept from the rows still to come.  Whole chain, f16: 8192 x 8192 x 256
+// 110 us from the first row on, 97 so; 4096 x 12000 x 64 79 and 67.  (Ordinary stores in place of the
+// streaming ones are slower or the same from 4 MB of output on: 8192 x 8192 x 256 100.7 and 99.5 us,
+// 2048 x 4096 x 128 19.6 and 19.4, f32 2048 x 4096 x 128 23.7 and 23.2.)
+//
+// VECS vectors a thread are in flight: with many CTAs one, since 32 registers let eight of them share an
+// SM (four take 40: six), four where all are resident at once anyway.  One and four, f16: 512 x 8192 x
+// 256 14.5 and 13.8 us, 700 x 2568 x 128 12.6 and 11.8, 1000 x 3000 x 128 12.9 and 13.2, 4096 x 4096 x
+// 128 30.3 and 31.8, 16384 x 4096 x 64 100 and 106; f32 600 x 30000 x 128 47.6 and 42.5, 4096 x 4096 x
+// 128 37.0 and 38.4.
+template <int VECS>
 __global__ void __launch_bounds__(256)
 rescale_rows_kernel(void *__restrict__ out_v, int out_f32, int N, int64_t ld_out, int BN, int num_nb,
                     const float2 *__restrict__ tile_stats, const float2 *__restrict__ global_stats,
@@ -83,15 +90,15 @@ rescale_rows_kernel(void *__restrict__ out_v, int out_f32, int N, int64_t ld_out
     float *frow = static_cast<float *>(out_v) + row * ld_out;
     if ((N % 4 == 0) && (ld_out % 4 == 0) && ((reinterpret_cast<uintptr_t>(out_v) & 15) == 0) && (BN % 4 == 0)) {
       float4 *o4 = reinterpret_cast<float4 *>(frow);
-      for (int j0 = c0 / 4 + threadIdx.x; j0 < c1 / 4; j0 += kRescaleVecs * blockDim.x) {
-        float4 x[kRescaleVecs];
+      for (int j0 = c0 / 4 + threadIdx.x; j0 < c1 / 4; j0 += VECS * blockDim.x) {
+        float4 x[VECS];
 #pragma unroll
-        for (int u = 0; u < kRescaleVecs; ++u) {
+        for (int u = 0; u < VECS; ++u) {
           const int j = j0 + u * blockDim.x;
           if (j < c1 / 4) x[u] = o4[j];
         }
 #pragma unroll
-        for (int u = 0; u < kRescaleVecs; ++u) {
+        for (int u = 0; u < VECS; ++u) {
           const int j = j0 + u * blockDim.x;
           if (j < c1 / 4) {
             const float fct = factor[(j * 4) / BN];
@@ -109,15 +116,15 @@ rescale_rows_kernel(void *__restrict__ out_v, int out_f32, int N, int64_t ld_out
   const bool vec_ok = (N % 8 == 0) && (ld_out % 8 == 0) && ((reinterpret_cast<uintptr_t>(out) & 15) == 0) && (BN % 8 == 0);
   if (vec_ok) {
     uint4 *o4 = reinterpret_cast<uint4 *>(orow);
-    for (int j0 = c0 / 8 + threadIdx.x; j0 < c1 / 8; j0 += kRescaleVecs * blockDim.x) {
-      uint4 x[kRescaleVecs];
+    for (int j0 = c0 / 8 + threadIdx.x; j0 < c1 / 8; j0 += VECS * blockDim.x) {
+      uint4 x[VECS];
 #pragma unroll
-      for (int u = 0; u < kRescaleVecs; ++u) {
+      for (int u = 0; u < VECS; ++u) {
         const int j = j0 + u * blockDim.x;
         if (j < c1 / 8) x[u] = o4[j];
       }
 #pragma unroll
-      for (int u = 0; u < kRescaleVecs; ++u) {
+      for (int u = 0; u < VECS; ++u) {
         const int j = j0 + u * blockDim.x;
         if (j < c1 / 8) {
           const float f = factor[(j * 8) / BN];
@@ -199,8 +206,9 @@ cudaError_t launch_rescale_rows(void *out, int out_f32, int64_t rows, int N, int
   attr[0].val.programmaticStreamSerializationAllowed = 1;
   cfg.attrs = attr;
   cfg.numAttrs = 1;
-  return cudaLaunchKernelEx(&cfg, rescale_rows_kernel, out, out_f32, N, ld_out, BN, num_nb, tile_stats,
-                            global_stats, num_parts, rows, chunk);
+  constexpr int64_t kResident = 148 * 6;       // CTAs of the four-vector form that the chip holds at once
+  return cudaLaunchKernelEx(&cfg, rows * splits <= kResident ? rescale_rows_kernel<4> : rescale_rows_kernel<1>, out, out_f32, N, ld_out, BN,
+                            num_nb, tile_stats, global_stats, num_parts, rows, chunk);
 }
 
 // ---- operand copies -----------------------------------------------------------------------------
