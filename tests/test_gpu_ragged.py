@@ -80,8 +80,8 @@ def test_padded_rows_of_a_hide_what_lies_between_them(wtc_lib, cuda_dev):
     (1, 4000, 127, 33, "f16", {}),          # narrower than a tile, ragged K
     (1, 8200, 255, 63, "f32", {}),          # f32 probabilities, 256-column tile
     (4, 1021, 1021, 64, "f16", {}),
-    (24, 1021, 1021, 64, "f16", {}),        # relay: several tiles per CTA, two operand stages
-    (24, 700, 1001, 251, "f16", {}),        # relay with three stages, ragged K
+    (24, 1021, 1021, 64, "f16", {}),        # several tiles per CTA
+    (24, 700, 1001, 251, "f16", {}),        # the same, ragged K
     (24, 700, 1001, 251, "f16", {"shared": True}),
     (3, 200, 2047, 72, "f32", {}),          # full cluster of eight
     (1, 257, 2049, 64, "f16", {}),          # tiled: one column in the ninth tile
@@ -281,3 +281,37 @@ def test_f32_results_of_ragged_chains_are_no_further_off(wtc_lib, cuda_dev, M, N
             w.check_device_status()
             off[name] += float((got.double() - P).norm() / P.norm())
     assert off["tc"] <= off["simt"], off
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("batch,M,N,K", [(1, 4000, 1021, 601), (6, 500, 1001, 250), (1, 2500, 3001, 65)])
+def test_ragged_calls_on_host_buffers(wtc_lib, cuda_dev, batch, M, N, K):
+    """Slabs of a ragged call: rows of A and of the output off their 16-byte boundaries, one workspace for all of them."""
+    w = wtc_lib
+    A, B = _operands(batch, M, N, K)
+    for _ in range(2):
+        got = w.matmul_softmax_host(A, B, 0.1)
+        r = oracle.compare(got.reshape(-1, N), _ref(A, B, 0.1).reshape(-1, N))
+        assert r["ok"], r
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("M,N,K,kw", [(2000, 1021, 61, {}), (600, 3001, 64, {}), (2000, 1021, 64, {"ldb": 1024})])
+def test_operands_ready_with_ragged_rows(wtc_lib, cuda_dev, M, N, K, kw):
+    """The loads wait for the call's own copies (if it makes any), the stores for the call before: different operands through
+    one workspace into one output, back to back, leave the last call's result."""
+    import torch
+    w = wtc_lib
+    sets = [_operands(1, M, kw.get("ldb", N), K, seed=i) for i in range(5)]
+    dev = [(torch.from_numpy(A).to(cuda_dev), torch.from_numpy(B).to(cuda_dev)) for A, B in sets]
+    d = w.make_desc(1, M, N, K, scale=0.1, flags=w.FLAG_OPERANDS_READY, **kw)
+    ws = torch.empty(max(16, w.workspace_bytes(d)), device=cuda_dev, dtype=torch.uint8)
+    out = torch.empty((M, N), device=cuda_dev, dtype=torch.float16)
+    torch.cuda.synchronize()
+    for _ in range(10):
+        for A, B in dev:
+            assert w.lib().wtc_matmul_softmax_launch(C.byref(d), A.data_ptr(), B.data_ptr(), out.data_ptr(), ws.data_ptr(), ws.numel(), w.current_stream_ptr(), None) == 0
+    w.check_device_status()
+    A, B = sets[-1]
+    r = oracle.compare(out.cpu().numpy(), oracle.chain(A, np.ascontiguousarray(B[:, :N]), 0.1))
+    assert r["ok"], r
