@@ -32,6 +32,8 @@ def test_plans_describe_the_tile_kernel(wtc_lib):
     assert w.plan_query(d).launches == 2
     d.o_batch_stride = 301 * 4096
     assert w.plan_query(d).launches == 4
+    # so many rows that the last tile's would not fit 32 bits
+    assert fields(1, 2 ** 31 - 127, 1, 1)[5] == 0 and fields(1, 2 ** 31 - 129, 1, 1)[5] > 0
     # f16 output: rows of more than eight tiles stay with the row kernel
     assert w.plan_query(w.make_desc(1, 300, 4096, 1024, w.F32, w.F16)).stages == 0
 

@@ -490,7 +490,7 @@ int pick_tile(const SimtParams &p) {
 // 1024 x 1024 x 128: 35 against 14.5).  (R = 0: refused, rows longer than the row kernel takes.)  A row of
 // more than eight column tiles keeps its logits in the output, so that has to be f32.
 bool use_tiles(const SimtParams &p, int R) {
-  if (p.in_f16 || R == 0) return false;
+  if (p.in_f16 || R == 0 || p.M > 0x7fffffff - kTileChoices[0].bm) return false;      // (a tile's rows are counted in 32 bits)
   if (static_cast<double>(p.batch) * p.M * p.N * (p.K > 0 ? p.K : 1) < (1 << 23)) return false;
   return !p.out_f16 || p.N <= 8 * kTileChoices[pick_tile(p)].bn;
 }
