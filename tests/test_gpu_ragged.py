@@ -215,6 +215,17 @@ def test_plans_of_few_rows_against_a_wide_matrix(wtc_lib):
     assert p.kernel == w.KERNEL_TC_TILED and p.workspace_bytes == 16 * 33 * 8
 
 
+def test_small_operands_of_long_k_keep_wide_tiles(wtc_lib):
+    """Few rows against a wide matrix: 37 to 54 tiles of 256 columns, K beyond 2048 and A of less than 128 KB."""
+    w = wtc_lib
+    tile = lambda *shape: w.plan_query(w.make_desc(1, *shape)).tile_n
+    assert tile(2, 36 * 256 + 8, 2056) == 256 and tile(2, 54 * 256, 2056) == 256 and tile(15, 10240, 4096) == 256
+    assert tile(2, 36 * 256, 2056) == 128 and tile(2, 54 * 256 + 8, 2056) == 128
+    assert tile(2, 10240, 2048) == 128 and tile(16, 10240, 4096) == 128
+    p = w.plan_query(w.make_desc(1, 2, 10240, 4096))
+    assert p.workspace_bytes == w.workspace_bytes(w.make_desc(1, 2, 10240, 4096)) == 2 * 40 * 8
+
+
 def test_pairs_on_request_keep_their_tiles(wtc_lib):
     """WTC_FLAG_PAIR pairs CTAs whenever there are two row blocks: 256-column tiles, whatever the number of tiles."""
     w = wtc_lib

@@ -172,7 +172,10 @@ int resolve(const wtc_chain_desc *in, Resolved &r) {
   // 9.2 vs 11.1 us; but 2048x1024x1024 18.6 vs 14.5 us, where sixteen 8-CTA clusters need two rounds), and (c) for rows of
   // more columns than a cluster holds when there are at most 64 tiles of 256 columns: few rows against a wide matrix are
   // bound by how many SMs stream it (16x4096x8192 35.6 vs 53.2 us, 128x8192x2048 16.8 vs 22.0, 16x16000x8192 46.8 vs 59.6;
-  // beyond 64 the second column block of a CTA costs more than the idle SMs: 16x18944x512 14.3 vs 13.6).
+  // beyond 64 the second column block of a CTA costs more than the idle SMs: 16x18944x512 14.3 vs 13.6).  Not between 37 and
+  // 54 tiles of 256 when K is long and A small: the narrow tiles read A twice as often, and an A of less than 128 KB is read
+  // slowly (2x10240x4096 34.2 vs 32.8 us, 4x10240x2936 28.9 vs 26.3, 4x13152x2936 31.0 vs 28.8; but 16x10240x4096 23.8 vs 33.0,
+  // 2x8192x4096 1.03 times as fast, 2x16000x4096 1.07, 2x10240x2048 1.02).
   r.bn = wtc::kTcBlockN;
   r.narrow = false;
   if (d.tile_n == 128) r.bn = 128;
@@ -183,7 +186,8 @@ int resolve(const wtc_chain_desc *in, Resolved &r) {
     const int64_t nb128 = (d.N + 127) / 128, nb256 = (d.N + 255) / 256;
     if (d.N <= 128) r.bn = 128;
     else if (!(d.flags & WTC_FLAG_FORCE_TILED) && nb128 <= 8 && units * nb256 <= 74 && units <= kResident[nb128]) r.bn = 128;
-    else if (!(d.flags & (WTC_FLAG_FORCE_TILED | WTC_FLAG_PAIR)) && nb256 > 8 && units * nb256 <= 64) {      // (CTA pairs have 256-column tiles)
+    else if (!(d.flags & (WTC_FLAG_FORCE_TILED | WTC_FLAG_PAIR)) && nb256 > 8 && units * nb256 <= 64 &&      // (CTA pairs have 256-column tiles)
+             !(units * nb256 > 36 && units * nb256 <= 54 && d.K > 2048 && d.batch * d.M * d.K < 65536)) {
       r.bn = 128;
       r.narrow = true;
     }
