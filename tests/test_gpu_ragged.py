@@ -107,8 +107,8 @@ def test_ragged_matches_the_checker(wtc_lib, cuda_dev, batch, M, N, K, out, kw):
         r = oracle.compare(got.reshape(-1, N), _ref(A, B, scale).reshape(-1, N))
         assert r["ok"], r
     simt = w.matmul_softmax(tA, tB, scale, out_dtype=odt, acc_dtype=acc, flags=w.FLAG_FORCE_SIMT).cpu().numpy().astype(np.float64)
-    # both round the same f32 sums (differing by their order) to the output type: one ulp of it apart (2^-10 relative; two for the
-    # tiled form, which rounds twice), and with an f16 matmul result one ulp of a logit (2^-10 relative, |logit| < 8) besides
+    # both round the same f32 sums (differing by their order) to the output type: one ulp of it apart (2^-10 relative; twice that is
+    # allowed), and with an f16 matmul result one ulp of a logit (2^-10 relative, |logit| < 8) besides
     tol = (2.0 ** -9 if out == "f16" else 2e-5) + (2.0 ** -7 if acc == w.F16 else 0)
     assert (np.abs(got.astype(np.float64) - simt) <= tol * simt + 2.0 ** -23).all()
 

@@ -233,7 +233,7 @@ __device__ __forceinline__ float share_max(float extreme, float c2) { return fma
 // A share's exponents are 2^(v * c2 - m), one FMA a value.  The rounding of the maximum m is the same factor on all of the share's
 // values and cancels in the quotient; but when the logits lie so far from zero that it amounts to more than 2^8 (an f16 ends at
 // 2^16, an f32 at 2^128), c2 gives way to the power of two below it, whose product with the extreme is exact: neighbouring f32
-// sums are at least a factor of 2^16 apart there, whatever the factor.  Such shares take the forms' general path.  (The extreme
+// sums are still a factor of 2^8 and more apart then.  Such shares take the forms' general path.  (The extreme
 // is taken a second time there: kept in a register it costs every tile, 14.00 against 13.97 us for 4096 x 1024 x 1024.)
 __device__ __forceinline__ bool far_from_zero(float m) { return fabsf(m) >= 268435456.f && m > kLowest; }
 __device__ __forceinline__ float far_factor(float c2) { return __uint_as_float(__float_as_uint(c2) & 0xFF800000u); }

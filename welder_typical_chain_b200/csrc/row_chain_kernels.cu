@@ -384,7 +384,7 @@ cudaError_t launch_rows(const void *X, void *Out, int64_t rows, int N, int64_t l
   auto threads_for = [&](int n, int nv) { return (((n + nv * V - 1) / (nv * V)) + 31) & ~31; };
   const int t4 = threads_for(N, 4), t8 = threads_for(N, 8), t16 = threads_for(N, 16);
   if (t4 <= 512) {
-    // f16 rows beyond 12288: packed, three CTAs an SM instead of two (8192 x 16384: 90 against 107 us; 8192 x 10000: 61 against 55)
+    // f16 rows beyond 12288: packed, three CTAs an SM instead of two (8192 x 16384: 88 against 99 us; 8192 x 10000: 61 against 55)
     if (F16 && N > 12288) row_chain_cta_kernel<KIND, F16, 4, RAGGED, F16><<<g, t4, 0, s>>>(X, Out, N, ld_in, ld_out, c1, c2);
     else row_chain_cta_kernel<KIND, F16, 4, RAGGED, false><<<g, t4, 0, s>>>(X, Out, N, ld_in, ld_out, c1, c2);
     return cudaGetLastError();

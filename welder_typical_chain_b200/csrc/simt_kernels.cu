@@ -127,7 +127,7 @@ simt_fused_kernel(const void *__restrict__ A, const void *__restrict__ B, void *
 // probabilities are written once.  Rows of more than eight column tiles (f32 output): the tiles store
 // logits, and a row-softmax pass follows in place.
 // Bound by the FMA pipes: 4096 x 1024 x 1024 takes 186 us (46 TFLOP/s; the 128 tiles of this shape can reach
-// 64 of the chip's 74) where the row kernel, one column a thread, took 479 (every FMA there reads A from
+// 64 of the chip's 74) where the row kernel, one column a thread, took 564 (every FMA there reads A from
 // shared memory, and each row block reads B alone).  16 x 8 results a thread need six 16-byte reads of
 // shared memory for 64 two-wide FMAs.
 constexpr int kTileK = 16;
