@@ -129,7 +129,8 @@ const char *wtc_last_error(void);
 /* Resolve a descriptor to a kernel plan without touching the device. */
 int wtc_plan_query(const wtc_chain_desc *desc, wtc_plan_info *out);
 
-/* Scratch memory (global memory beyond inputs and outputs) a launch needs. */
+/* Scratch memory (global memory beyond inputs and outputs) a launch needs; at least the plan's figure, and more
+ * where pointers off their 16-byte boundaries are copied into rows on them. */
 int wtc_matmul_softmax_workspace_bytes(const wtc_chain_desc *desc, size_t *bytes);
 
 /*

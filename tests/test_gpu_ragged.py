@@ -75,6 +75,36 @@ def test_padded_rows_of_a_hide_what_lies_between_them(wtc_lib, cuda_dev):
 
 
 @pytest.mark.gpu
+@pytest.mark.parametrize("N,K,lda", [(1000, 61, 64), (1001, 61, 72), (3001, 65, 72)])
+def test_columns_of_a_wider_matrix_as_a(wtc_lib, cuda_dev, N, K, lda):
+    """A from the second column of wider rows on, two bytes behind a boundary: copied where the workspace has the room that
+    wtc_matmul_softmax_workspace_bytes asks for, and then the bits are those of the same A on its boundary."""
+    import torch
+    w = wtc_lib
+    M = 700
+    A, B = _operands(1, M, N, K)
+    wide = torch.full((M, lda), float("nan"), device=cuda_dev, dtype=torch.float16)
+    wide[:, 1:1 + K] = torch.from_numpy(A).to(cuda_dev)
+    tA = torch.full((M, lda), float("nan"), device=cuda_dev, dtype=torch.float16)
+    tA[:, :K] = wide[:, 1:1 + K]
+    tB = torch.from_numpy(B).to(cuda_dev)
+    d = w.make_desc(1, M, N, K, scale=0.1, lda=lda)
+    need, planned = w.workspace_bytes(d), w.plan_query(d).workspace_bytes
+    assert need == planned + -(-M * ((K + 7) // 8 * 8) * 2 // 256) * 256
+    got = []
+    for ptr, size in ((tA.data_ptr(), planned), (wide.data_ptr() + 2, need), (wide.data_ptr() + 2, planned)):
+        ws = torch.full((size + 256,), 0x7f, device=cuda_dev, dtype=torch.uint8)
+        out = torch.empty((M, N), device=cuda_dev, dtype=torch.float16)
+        assert w.lib().wtc_matmul_softmax_launch(C.byref(d), ptr, tB.data_ptr(), out.data_ptr(), ws.data_ptr(), size, w.current_stream_ptr(), None) == 0
+        w.check_device_status()
+        assert bool((ws[size:] == 0x7f).all())
+        got.append(out)
+    assert torch.equal(got[0], got[1])
+    r = oracle.compare(got[2].cpu().numpy(), oracle.chain(A, B, 0.1))      # (the SIMT kernel)
+    assert r["ok"], r
+
+
+@pytest.mark.gpu
 @pytest.mark.parametrize("batch,M,N,K,out,kw", [
     (1, 2000, 129, 64, "f16", {}),          # 128-column tiles, one column in the second
     (1, 4000, 127, 33, "f16", {}),          # narrower than a tile, ragged K

@@ -70,6 +70,8 @@ struct Resolved {
   // copies in the workspace (copy_a / copy_b: their bytes, 0 = read in place), output rows written by the epilogue
   bool ragged;
   size_t copy_a, copy_b;
+  // ... and the bytes of a copy of A that only a pointer off its 16-byte boundary needs (else the SIMT kernel takes the call)
+  size_t spare_a;
   bool direct_out;
   // ... of the tiled flavour with f16 output: these chains round a probability once, as the SIMT kernel does, so no values relative
   // to a tile's maximum are stored on the way; the tiles' statistics come from a first pass over the contraction, the
@@ -147,6 +149,7 @@ int resolve(const wtc_chain_desc *in, Resolved &r) {
     const wtc_chain_desc outer = d;
     const bool bb = r.b_batched;
     r = ri;
+    r.spare_a = 0;            // (the rounded copies lie on their boundaries)
     r.d = outer;
     r.b_batched = bb;
     r.inner = inner;
@@ -220,7 +223,7 @@ int resolve(const wtc_chain_desc *in, Resolved &r) {
   // Only what the SIMT kernel takes too (its row of logits in shared memory), since a call without the workspace, or with
   // pointers off their 16-byte boundaries, runs there.
   const bool tiled_row = r.num_nb > 8 || (d.flags & WTC_FLAG_FORCE_TILED);
-  r.copy_a = r.copy_b = 0;
+  r.copy_a = r.copy_b = r.spare_a = 0;
   r.direct_out = r.two_pass = false;
   r.sum_kb = 0;
   r.ragged = !tc_shape && d.in_dtype == WTC_F16 && d.M > 0 && d.N > 0 && d.K > 0 && d.variant == WTC_VARIANT_FUSED &&
@@ -232,7 +235,9 @@ int resolve(const wtc_chain_desc *in, Resolved &r) {
     r.num_rb = static_cast<int>((d.M + wtc::kTcBlockM - 1) / wtc::kTcBlockM);
     r.num_kb = static_cast<int>((d.K + r.kd - 1) / r.kd);
     // (strides count: a K that is no multiple of 8 is only an extent of A's map, which fills zeros behind it)
-    if (!mult8(d.lda) || !mult8(d.a_batch_stride)) r.copy_a = align256(static_cast<size_t>(d.batch) * d.M * round8(d.K) * 2);
+    const size_t bytes_a = align256(static_cast<size_t>(d.batch) * d.M * round8(d.K) * 2);
+    if (!mult8(d.lda) || !mult8(d.a_batch_stride)) r.copy_a = bytes_a;
+    else if (!mult8(d.K)) r.spare_a = bytes_a;
     if (!mult8(d.ldb) || !mult8(d.b_batch_stride)) r.copy_b = align256(static_cast<size_t>(r.b_batched ? d.batch : 1) * d.K * round64(d.N) * 2);
     r.two_pass = tiled_row && d.out_dtype == WTC_F16;
     r.sum_kb = d.out_dtype == WTC_F32 && r.num_kb > kRaggedSumKb ? kRaggedSumKb : 0;
@@ -528,29 +533,31 @@ int launch_resolved(Resolved &r, const void *A, const void *B, void *Out, void *
     return e == cudaSuccess ? WTC_OK : cuda_fail(e, "unfused tensor-core pipeline launch");
   }
 
-  const bool ws_ok = !r.ragged || r.plan.workspace_bytes == 0 || (ws && ws_bytes >= r.plan.workspace_bytes && aligned16(ws));
-  const bool ptr_ok = (r.copy_a || aligned16(A)) && (r.copy_b || aligned16(B)) && (r.direct_out || aligned16(Out)) && ws_ok;
+  const size_t spare_a = r.spare_a && !aligned16(A) && ws_bytes >= r.plan.workspace_bytes + r.spare_a ? r.spare_a : 0;
+  const size_t ragged_ws = r.plan.workspace_bytes + spare_a, copy_a = r.copy_a + spare_a;      // (one of the two is 0)
+  const bool ws_ok = !r.ragged || ragged_ws == 0 || (ws && ws_bytes >= ragged_ws && aligned16(ws));
+  const bool ptr_ok = (copy_a || aligned16(A)) && (r.copy_b || aligned16(B)) && (r.direct_out || aligned16(Out)) && ws_ok;
   bool tiled = r.plan.kernel == WTC_KERNEL_TC_TILED || (mode == 1 && r.tc_ok);
   if ((r.plan.kernel == WTC_KERNEL_TC_CLUSTER || tiled) && ptr_ok) {
     const int sms = num_sms();
     if (sms <= 0) return fail(WTC_E_CUDA, "no usable CUDA device");
     int64_t lda = d.lda, a_batch_stride = d.a_batch_stride;
-    if (r.copy_a || r.copy_b) {
+    if (copy_a || r.copy_b) {
       unsigned char *base = static_cast<unsigned char *>(ws);
       wtc::OperandCopy ca{}, cb{};
-      if (r.copy_a) {
+      if (copy_a) {
         ca = wtc::OperandCopy{A, base, d.batch, d.M, d.K, d.lda, d.a_batch_stride, round8(d.K)};
         A = base;
         lda = round8(d.K); a_batch_stride = d.M * lda;
       }
       if (r.copy_b) {
-        cb = wtc::OperandCopy{B, base + r.copy_a, r.b_batched ? d.batch : 1, d.K, d.N, d.ldb, r.b_batched ? d.b_batch_stride : 0, round64(d.N)};
-        B = base + r.copy_a;
+        cb = wtc::OperandCopy{B, base + copy_a, r.b_batched ? d.batch : 1, d.K, d.N, d.ldb, r.b_batched ? d.b_batch_stride : 0, round64(d.N)};
+        B = base + copy_a;
       }
       const cudaError_t e = wtc::launch_copy_operands(ca, cb, false, s);
       if (e != cudaSuccess) return cuda_fail(e, "operand copy launch");
-      ws = base + r.copy_a + r.copy_b;
-      ws_bytes -= r.copy_a + r.copy_b;
+      ws = base + copy_a + r.copy_b;
+      ws_bytes -= copy_a + r.copy_b;
     }
     CUtensorMap tmA, tmB, tmO;
     // A's box is one swizzle span wide at most: 64 columns (a 128-deep stage takes two), or 32 with the 64-byte swizzle
@@ -582,7 +589,7 @@ int launch_resolved(Resolved &r, const void *A, const void *B, void *Out, void *
     p.timeline = g_timeline ? g_timeline + static_cast<size_t>(g_timeline_launch++ % 4) * 148 * 48 : nullptr;
 #endif
     p.use_pdl = g_use_pdl;
-    p.operands_ready = (d.flags & WTC_FLAG_OPERANDS_READY) && !r.copy_a && !r.copy_b ? 1 : 0;   // (the copies are earlier work on the stream)
+    p.operands_ready = (d.flags & WTC_FLAG_OPERANDS_READY) && !copy_a && !r.copy_b ? 1 : 0;   // (the copies are earlier work on the stream)
     p.out_f32 = out32;
     p.direct_out = r.direct_out;
     p.sum_kb = r.sum_kb;
@@ -653,7 +660,7 @@ int wtc_matmul_softmax_workspace_bytes(const wtc_chain_desc *desc, size_t *bytes
   Resolved r;
   int rc = resolve(desc, r);
   if (rc) return rc;
-  size_t need = r.plan.workspace_bytes;
+  size_t need = r.plan.workspace_bytes + r.spare_a;      // (a launch with A on its boundary does with the plan's bytes)
   // the sharded form always runs the tiled schedule
   if (r.tc_ok) {
     const size_t tiled = static_cast<size_t>(r.d.batch) * r.d.M * r.num_nb * sizeof(float2);
