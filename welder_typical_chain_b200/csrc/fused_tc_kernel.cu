@@ -42,7 +42,7 @@
 // OUT32: f32 probabilities.
 // DIRECT: output rows that TMA cannot store (a stride that is no multiple of 16 bytes): the warp
 // that staged a tile writes its rows itself (split form).  Tiled with f16 output it runs twice, statistics
-// first (TcParams::stats_pass), so that a probability is rounded once.
+// first (TcParams::stats_pass), so that a probability is rounded once.  DIRECT = 2 (f32 output): long K in partial sums.
 // KD, TM: K depth of a pipeline stage (64; 32 or 128 on request) and rows of a tile (128;
 // 64 on request, tcgen05.mma with M = 64) -- the schedule's tileK and tileM.
 //
@@ -307,7 +307,7 @@ __device__ __forceinline__ void scale_pack(const uint32_t (&r)[32], float f, uin
   for (int i = 0; i < 32; i += 2) h[i >> 1] = pack_f16x2(__uint_as_float(r[i]) * f, __uint_as_float(r[i + 1]) * f);
 }
 
-template <int BN, int STAGES, bool CLUSTER, int EPI, bool PAIR, bool OUT32, int KD, int TM, bool DIRECT>
+template <int BN, int STAGES, bool CLUSTER, int EPI, bool PAIR, bool OUT32, int KD, int TM, int DIRECT>
 __global__ void __launch_bounds__(kThreadsFor(EPI), 1)
 fused_tc_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CUtensorMap tmB,
                 const __grid_constant__ CUtensorMap tmO, const TcParams p) {
@@ -320,13 +320,15 @@ fused_tc_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__
   constexpr bool TWO_PASS = DIRECT && !CLUSTER && !OUT32;   // p.stats_pass
   // Partial sums (p.sum_kb): the tensor core's running f32 sum loses a little with every step, and beyond some 256 products more
   // than FMAs do (K = 1023: 1.7e-6 of the result against 1.05e-6).  Added in registers, sums of 256 keep the error below theirs.
-  constexpr bool PARTIAL = DIRECT && OUT32;
+  // (Instances of their own: as a branch of every DIRECT one they cost 3000 x 777 x 128 with f32 output 12.44 instead of 11.94 us.)
+  constexpr bool PARTIAL = DIRECT == 2;
   constexpr int HC = L::kHalfCols;      // columns per epilogue thread
   constexpr int NCH = HC / 32;          // 32-column chunks per epilogue thread
   constexpr int kEpiThreads = (RELAY || SINGLE) ? 512 : 256;
   static_assert(!(RELAY || SINGLE) || (CLUSTER && !PAIR && !OUT32 && BN == 256 && TM == 128), "sixteen-warp epilogues: cluster flavour, 128 x 256 tiles, f16 staged stores");
   static_assert(!OUT32 || !PAIR, "f32 output: unpaired CTAs");
   static_assert(!PAIR || !CLUSTER, "CTA pairs: tiled flavour only");
+  static_assert(!PARTIAL || OUT32, "partial sums: f32 output");
   static_assert(!DIRECT || (!PAIR && EPI == EPI_SPLIT && KD == kTcBlockK && TM == kTcBlockM), "rows written by threads: split form, default tiles");
   // The 128-byte swizzle needs the stage buffers on 1024-byte boundaries.  There is no
   // static shared memory in this kernel, so the dynamic window starts aligned; if it ever
@@ -1232,7 +1234,7 @@ struct DeviceFacts {
   int registers = 0;
 };
 
-template <int BN, int STAGES, bool CLUSTER, int EPI, bool PAIR, bool OUT32, int KD, int TM, bool DIRECT>
+template <int BN, int STAGES, bool CLUSTER, int EPI, bool PAIR, bool OUT32, int KD, int TM, int DIRECT>
 cudaError_t launch_impl(const CUtensorMap &tmA, const CUtensorMap &tmB, const CUtensorMap &tmO, TcParams p,
                         int cluster_n, int num_sms, cudaStream_t s, TcLaunchInfo *info) {
   using L = SmemLayout<BN, STAGES, CLUSTER, EPI, PAIR, OUT32, KD, TM>;
@@ -1304,28 +1306,31 @@ cudaError_t launch_impl(const CUtensorMap &tmA, const CUtensorMap &tmB, const CU
 
 // Every instantiated variant, once: X(BN, STAGES, CLUSTER, EPI, PAIR, OUT32, KD, TM, DIRECT).
 #define WTC_TC_VARIANTS(X)                                                                                \
-  X(128, 4, true, EPI_SPLIT, false, true, 64, 128, false) X(kTcBlockN, 3, true, EPI_SPLIT, false, true, 64, 128, false)            \
-  X(128, 4, true, EPI_SPLIT, false, false, 64, 128, false) X(kTcBlockN, 3, true, EPI_SPLIT, false, false, 64, 128, false)          \
-  X(kTcBlockN, 2, true, EPI_RELAY, false, false, 64, 128, false) X(kTcBlockN, 3, true, EPI_RELAY, false, false, 64, 128, false)    \
-  X(kTcBlockN, 4, true, EPI_SINGLE, false, false, 64, 128, false)                                                      \
-  X(128, 6, false, EPI_SPLIT, false, true, 64, 128, false) X(kTcBlockN, 4, false, EPI_SPLIT, false, true, 64, 128, false)          \
-  X(128, 6, false, EPI_SPLIT, false, false, 64, 128, false) X(kTcBlockN, 4, false, EPI_SPLIT, false, false, 64, 128, false)        \
-  X(kTcBlockN, 6, false, EPI_SPLIT, true, false, 64, 128, false)                                                       \
+  X(128, 4, true, EPI_SPLIT, false, true, 64, 128, 0) X(kTcBlockN, 3, true, EPI_SPLIT, false, true, 64, 128, 0)            \
+  X(128, 4, true, EPI_SPLIT, false, false, 64, 128, 0) X(kTcBlockN, 3, true, EPI_SPLIT, false, false, 64, 128, 0)          \
+  X(kTcBlockN, 2, true, EPI_RELAY, false, false, 64, 128, 0) X(kTcBlockN, 3, true, EPI_RELAY, false, false, 64, 128, 0)    \
+  X(kTcBlockN, 4, true, EPI_SINGLE, false, false, 64, 128, 0)                                                      \
+  X(128, 6, false, EPI_SPLIT, false, true, 64, 128, 0) X(kTcBlockN, 4, false, EPI_SPLIT, false, true, 64, 128, 0)          \
+  X(128, 6, false, EPI_SPLIT, false, false, 64, 128, 0) X(kTcBlockN, 4, false, EPI_SPLIT, false, false, 64, 128, 0)        \
+  X(kTcBlockN, 6, false, EPI_SPLIT, true, false, 64, 128, 0)                                                       \
   /* other stage depths (the schedule's tileK): eight-warp epilogue, f16 output */                        \
-  X(128, 8, true, EPI_SPLIT, false, false, 32, 128, false) X(kTcBlockN, 6, true, EPI_SPLIT, false, false, 32, 128, false)          \
-  X(128, 12, false, EPI_SPLIT, false, false, 32, 128, false) X(kTcBlockN, 8, false, EPI_SPLIT, false, false, 32, 128, false)       \
-  X(128, 2, true, EPI_SPLIT, false, false, 128, 128, false)                                                            \
-  X(128, 3, false, EPI_SPLIT, false, false, 128, 128, false) X(kTcBlockN, 2, false, EPI_SPLIT, false, false, 128, 128, false)       \
+  X(128, 8, true, EPI_SPLIT, false, false, 32, 128, 0) X(kTcBlockN, 6, true, EPI_SPLIT, false, false, 32, 128, 0)          \
+  X(128, 12, false, EPI_SPLIT, false, false, 32, 128, 0) X(kTcBlockN, 8, false, EPI_SPLIT, false, false, 32, 128, 0)       \
+  X(128, 2, true, EPI_SPLIT, false, false, 128, 128, 0)                                                            \
+  X(128, 3, false, EPI_SPLIT, false, false, 128, 128, 0) X(kTcBlockN, 2, false, EPI_SPLIT, false, false, 128, 128, 0)       \
   /* 64-row tiles (the schedule's tileM = 64), stage depth 32 or 64 */                                         \
-  X(128, 4, true, EPI_SPLIT, false, false, 64, 64, false) X(kTcBlockN, 3, true, EPI_SPLIT, false, false, 64, 64, false)      \
-  X(128, 6, false, EPI_SPLIT, false, false, 64, 64, false) X(kTcBlockN, 4, false, EPI_SPLIT, false, false, 64, 64, false)    \
-  X(128, 8, true, EPI_SPLIT, false, false, 32, 64, false) X(kTcBlockN, 6, true, EPI_SPLIT, false, false, 32, 64, false)      \
-  X(128, 12, false, EPI_SPLIT, false, false, 32, 64, false) X(kTcBlockN, 8, false, EPI_SPLIT, false, false, 32, 64, false) \
+  X(128, 4, true, EPI_SPLIT, false, false, 64, 64, 0) X(kTcBlockN, 3, true, EPI_SPLIT, false, false, 64, 64, 0)      \
+  X(128, 6, false, EPI_SPLIT, false, false, 64, 64, 0) X(kTcBlockN, 4, false, EPI_SPLIT, false, false, 64, 64, 0)    \
+  X(128, 8, true, EPI_SPLIT, false, false, 32, 64, 0) X(kTcBlockN, 6, true, EPI_SPLIT, false, false, 32, 64, 0)      \
+  X(128, 12, false, EPI_SPLIT, false, false, 32, 64, 0) X(kTcBlockN, 8, false, EPI_SPLIT, false, false, 32, 64, 0) \
   /* output rows that TMA cannot store */                                                                       \
-  X(128, 4, true, EPI_SPLIT, false, true, 64, 128, true) X(kTcBlockN, 3, true, EPI_SPLIT, false, true, 64, 128, true)    \
-  X(128, 4, true, EPI_SPLIT, false, false, 64, 128, true) X(kTcBlockN, 3, true, EPI_SPLIT, false, false, 64, 128, true)  \
-  X(128, 6, false, EPI_SPLIT, false, true, 64, 128, true) X(kTcBlockN, 4, false, EPI_SPLIT, false, true, 64, 128, true)  \
-  X(128, 6, false, EPI_SPLIT, false, false, 64, 128, true) X(kTcBlockN, 4, false, EPI_SPLIT, false, false, 64, 128, true)
+  X(128, 4, true, EPI_SPLIT, false, true, 64, 128, 1) X(kTcBlockN, 3, true, EPI_SPLIT, false, true, 64, 128, 1)    \
+  X(128, 4, true, EPI_SPLIT, false, false, 64, 128, 1) X(kTcBlockN, 3, true, EPI_SPLIT, false, false, 64, 128, 1)  \
+  X(128, 6, false, EPI_SPLIT, false, true, 64, 128, 1) X(kTcBlockN, 4, false, EPI_SPLIT, false, true, 64, 128, 1)  \
+  X(128, 6, false, EPI_SPLIT, false, false, 64, 128, 1) X(kTcBlockN, 4, false, EPI_SPLIT, false, false, 64, 128, 1) \
+  /* ... with f32 output and long K */ \
+  X(128, 4, true, EPI_SPLIT, false, true, 64, 128, 2) X(kTcBlockN, 3, true, EPI_SPLIT, false, true, 64, 128, 2)    \
+  X(128, 6, false, EPI_SPLIT, false, true, 64, 128, 2) X(kTcBlockN, 4, false, EPI_SPLIT, false, true, 64, 128, 2)
 
 // Form choice.  Cluster flavour: f32 probabilities and 128-column tiles take the split
 // epilogue; 256-column f16 tiles take the relay when a CTA sees several tiles (its two groups
@@ -1341,11 +1346,11 @@ bool tc_stage_depth_legal(bool tiled, int bn, bool out_f32, int kd, int tm) {
 }
 
 TcVariant tc_choose_variant(bool tiled, int bn, bool out_f32, int batch, int num_rb, int num_kb, int cluster_n,
-                            int epilogue_mode, int pair_mode, int num_sms, int resident, int kd, int tm, bool direct) {
+                            int epilogue_mode, int pair_mode, int num_sms, int resident, int kd, int tm, int direct) {
   if (direct) {
     // split form, no CTA pairs, default tiles (as a relay, whose storing warps are fewer: 47 against 42 us for 24504 x 1021 x 64)
     TcVariant v = tc_choose_variant(tiled, bn, out_f32, batch, num_rb, num_kb, cluster_n, kEpilogueSplit, 1, num_sms, 0);
-    v.direct = 1;
+    v.direct = direct;
     return v;
   }
   if ((kd != kTcBlockK || tm != kTcBlockM) && tc_stage_depth_legal(tiled, bn, out_f32, kd, tm)) {
@@ -1374,7 +1379,7 @@ TcVariant tc_choose_variant(bool tiled, int bn, bool out_f32, int batch, int num
 
 int tc_variant_smem_bytes(const TcVariant &v) {
 #define X(BN, ST, CL, EP, PA, O32, KD, TM, DI) \
-  if (v.bn == BN && v.stages == ST && (v.cluster != 0) == CL && v.epi == EP && (v.pair != 0) == PA && (v.out32 != 0) == O32 && v.kd == KD && v.tm == TM && (v.direct != 0) == DI) \
+  if (v.bn == BN && v.stages == ST && (v.cluster != 0) == CL && v.epi == EP && (v.pair != 0) == PA && (v.out32 != 0) == O32 && v.kd == KD && v.tm == TM && v.direct == DI) \
     return SmemLayout<BN, ST, CL, EP, PA, O32, KD, TM>::kDynamic;
   WTC_TC_VARIANTS(X)
 #undef X
@@ -1387,7 +1392,7 @@ namespace {
 cudaError_t launch_variant(const TcVariant &v, const CUtensorMap &tmA, const CUtensorMap &tmB, const CUtensorMap &tmO,
                            const TcParams &p, int cluster_n, int num_sms, cudaStream_t s, TcLaunchInfo *info) {
 #define X(BN, ST, CL, EP, PA, O32, KD, TM, DI) \
-  if (v.bn == BN && v.stages == ST && (v.cluster != 0) == CL && v.epi == EP && (v.pair != 0) == PA && (v.out32 != 0) == O32 && v.kd == KD && v.tm == TM && (v.direct != 0) == DI) \
+  if (v.bn == BN && v.stages == ST && (v.cluster != 0) == CL && v.epi == EP && (v.pair != 0) == PA && (v.out32 != 0) == O32 && v.kd == KD && v.tm == TM && v.direct == DI) \
     return launch_impl<BN, ST, CL, EP, PA, O32, KD, TM, DI>(tmA, tmB, tmO, p, cluster_n, num_sms, s, info);
   WTC_TC_VARIANTS(X)
 #undef X
@@ -1403,7 +1408,7 @@ cudaError_t launch_fused_cluster(const CUtensorMap &tmA, const CUtensorMap &tmB,
   // (before launching) when the clusters do not all fit the chip at once, and the split form runs
   TcVariant v = tc_choose_variant(false, bn, p.out_f32 != 0, p.batch, p.num_rb, p.num_kb, cluster_n, p.epilogue_mode, p.pair_mode,
                                   num_sms, /*resident=*/1 << 30, p.stage_k ? p.stage_k : kTcBlockK, p.tile_rows ? p.tile_rows : kTcBlockM,
-                                  p.direct_out != 0);
+                                  p.direct_out);
   if (v.epi == EPI_SINGLE) {
     const cudaError_t e = launch_variant(v, tmA, tmB, tmO, p, cluster_n, num_sms, s, info);
     if (e != cudaErrorNotSupported) return e;
@@ -1415,7 +1420,7 @@ cudaError_t launch_fused_cluster(const CUtensorMap &tmA, const CUtensorMap &tmB,
 cudaError_t launch_tiled_partial(const CUtensorMap &tmA, const CUtensorMap &tmB, const CUtensorMap &tmO,
                                  const TcParams &p, int bn, int num_sms, cudaStream_t s, TcLaunchInfo *info) {
   const TcVariant v = tc_choose_variant(true, bn, p.out_f32 != 0, p.batch, p.num_rb, p.num_kb, 1, p.epilogue_mode, p.pair_mode, num_sms, 0,
-                                        p.stage_k ? p.stage_k : kTcBlockK, p.tile_rows ? p.tile_rows : kTcBlockM, p.direct_out != 0);
+                                        p.stage_k ? p.stage_k : kTcBlockK, p.tile_rows ? p.tile_rows : kTcBlockM, p.direct_out);
   return launch_variant(v, tmA, tmB, tmO, p, 1, num_sms, s, info);
 }
 

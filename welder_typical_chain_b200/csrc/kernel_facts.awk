@@ -3,7 +3,7 @@
 # one per instantiated variant of the kernel template (the template arguments are read off
 # the mangled entry name).
 /Compiling entry function/ {
-  have = match($0, /fused_tc_kernelILi[0-9]+ELi[0-9]+ELb[01]ELi[0-9]+ELb[01]ELb[01]ELi[0-9]+ELi[0-9]+ELb[01]E/)
+  have = match($0, /fused_tc_kernelILi[0-9]+ELi[0-9]+ELb[01]ELi[0-9]+ELb[01]ELb[01]ELi[0-9]+ELi[0-9]+ELi[0-9]+E/)
   if (have) {
     name = substr($0, RSTART, RLENGTH)
     n = split(name, part, /ELi|ELb|ILi|E$/)

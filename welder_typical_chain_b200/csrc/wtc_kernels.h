@@ -58,13 +58,13 @@ struct TcVariant {
   int bn, stages, cluster, epi, pair, out32;
   int kd;    // K depth of one pipeline stage: 64, or the schedule's tileK when it is 32 or 128 and legal
   int tm;    // rows of a tile: 128, or the schedule's tileM when it is 64 and legal
-  int direct = 0;   // the output rows are written by the epilogue's threads instead of TMA stores
+  int direct = 0;   // 1: the output rows are written by the epilogue's threads instead of TMA stores; 2: and K is summed in parts (f32 output)
 };
 // The variant the launchers below take for a call, worked out without a device: `resident` is how
 // many clusters of `cluster_n` CTAs the chip holds at once (the launchers ask the runtime; a plan
 // made without a device uses the figures measured on a 148-SM part).
 TcVariant tc_choose_variant(bool tiled, int bn, bool out_f32, int batch, int num_rb, int num_kb, int cluster_n,
-                            int epilogue_mode, int pair_mode, int num_sms, int resident, int kd = 64, int tm = 128, bool direct = false);
+                            int epilogue_mode, int pair_mode, int num_sms, int resident, int kd = 64, int tm = 128, int direct = 0);
 // Whether this stage depth and tile height have a kernel for this flavour, column tile and output type.
 bool tc_stage_depth_legal(bool tiled, int bn, bool out_f32, int kd, int tm = 128);
 // Dynamic shared memory and threads per CTA of a variant (0 if it is not instantiated).

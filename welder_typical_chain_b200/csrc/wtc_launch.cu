@@ -51,7 +51,7 @@ const KernelFacts kKernelFacts[] = {
 };
 const KernelFacts *facts_of(const wtc::TcVariant &v) {
   for (const KernelFacts &f : kKernelFacts)
-    if (f.bn == v.bn && f.stages == v.stages && f.cluster == (v.cluster != 0) && f.epi == v.epi && f.pair == (v.pair != 0) && f.out32 == (v.out32 != 0) && f.kd == v.kd && f.tm == v.tm && f.direct == (v.direct != 0))
+    if (f.bn == v.bn && f.stages == v.stages && f.cluster == (v.cluster != 0) && f.epi == v.epi && f.pair == (v.pair != 0) && f.out32 == (v.out32 != 0) && f.kd == v.kd && f.tm == v.tm && f.direct == v.direct)
       return &f;
   return nullptr;
 }
@@ -72,7 +72,7 @@ struct Resolved {
   size_t copy_a, copy_b;
   // ... and the bytes of a copy of A that only a pointer off its 16-byte boundary needs (else the SIMT kernel takes the call)
   size_t spare_a;
-  bool direct_out;
+  int direct_out;         // (2: with partial sums)
   // ... of the tiled flavour with f16 output: these chains round a probability once, as the SIMT kernel does, so no values relative
   // to a tile's maximum are stored on the way; the tiles' statistics come from a first pass over the contraction, the
   // probabilities from a second (error against 64 bits 2.1e-4 of the result; with f16 values rescaled 2.7e-4)
@@ -224,8 +224,8 @@ int resolve(const wtc_chain_desc *in, Resolved &r) {
   // pointers off their 16-byte boundaries, runs there.
   const bool tiled_row = r.num_nb > 8 || (d.flags & WTC_FLAG_FORCE_TILED);
   r.copy_a = r.copy_b = r.spare_a = 0;
-  r.direct_out = r.two_pass = false;
-  r.sum_kb = 0;
+  r.direct_out = r.sum_kb = 0;
+  r.two_pass = false;
   r.ragged = !tc_shape && d.in_dtype == WTC_F16 && d.M > 0 && d.N > 0 && d.K > 0 && d.variant == WTC_VARIANT_FUSED &&
              !(d.flags & WTC_FLAG_FORCE_SIMT) && static_cast<double>(d.batch) * d.M * d.N * d.K >= kRaggedMinWork &&
              wtc::simt_fused_takes(simt_params(r)) && static_cast<int64_t>(d.batch) * r.num_rb * r.num_nb < 0x7fffffff &&
@@ -241,7 +241,8 @@ int resolve(const wtc_chain_desc *in, Resolved &r) {
     if (!mult8(d.ldb) || !mult8(d.b_batch_stride)) r.copy_b = align256(static_cast<size_t>(r.b_batched ? d.batch : 1) * d.K * round64(d.N) * 2);
     r.two_pass = tiled_row && d.out_dtype == WTC_F16;
     r.sum_kb = d.out_dtype == WTC_F32 && r.num_kb > kRaggedSumKb ? kRaggedSumKb : 0;
-    r.direct_out = !mult8(d.N) || !mult8(d.ldo) || !mult8(d.o_batch_stride) || r.two_pass || r.sum_kb;      // (a TMA store fills the last 16 bytes of a row)
+    // (a TMA store fills the last 16 bytes of a row)
+    r.direct_out = r.sum_kb ? 2 : !mult8(d.N) || !mult8(d.ldo) || !mult8(d.o_batch_stride) || r.two_pass ? 1 : 0;
   }
 
   if (d.variant == WTC_VARIANT_BASELINE) {
